@@ -99,8 +99,9 @@ struct tbfp_handle {
   // flow control: dxc(1..nx), dyf(1..ny), dzf(1..nz) on the device, ny*nz row partials + the sum
   double *d_fdxc = nullptr, *d_fdyf = nullptr, *d_fdzf = nullptr, *d_fpart = nullptr;
   // surface tension (tbfp_surface_tension): tables and dense scratch, made on first use
-  double *d_st_dyc = nullptr, *d_st_yf = nullptr, *d_st_cp = nullptr, *d_st_kap = nullptr, *h_kap = nullptr;
+  double *d_st_dyc = nullptr, *d_st_yf = nullptr, *d_st_kap = nullptr, *h_kap = nullptr;
   unsigned char *d_st_fl = nullptr;
+  int *d_st_list = nullptr, *d_st_count = nullptr;  // the mixed cells of the last call
   MgSolver *mg = nullptr;   // MG_MODE hierarchy (tbfp_pcg_setup)
   std::vector<double> mdxf, mdxc, mdyf, mdyc, mdzf, mdzc;  // caller's metrics, kept for tbfp_pcg_setup
   double *h_beta = nullptr, *h_q = nullptr;                // device copies for tbfp_pcg_solve
@@ -1699,7 +1700,7 @@ int tbfp_surface_tension_dev(tbfp_handle *h, const double *c, double sigma, doub
   if (!std::isfinite(sigma)) return set_err(h, TBFP_EINVAL, "tbfp_surface_tension: sigma must be finite");
   cudaSetDevice(h->device);
   const long n = (long)h->nx * h->ny * h->nz;
-  if (!h->d_st_cp) {
+  if (!h->d_st_count) {  // allocated last
     std::vector<double> dyc(h->mdyc.begin(), h->mdyc.end()), yf(h->ny + 1, 0.0);
     double acc = 0.0;
     for (int m = 0; m < h->ny; ++m) {  // face positions: sequential sums of dyf
@@ -1707,8 +1708,8 @@ int tbfp_surface_tension_dev(tbfp_handle *h, const double *c, double sigma, doub
       yf[m + 1] = acc;
     }
     if ((rc = upload(h, &h->d_st_dyc, dyc)) || (rc = upload(h, &h->d_st_yf, yf)) ||
-        (rc = dev_alloc(h, &h->d_st_cp, (size_t)n)) || (rc = dev_alloc(h, &h->d_st_kap, (size_t)n)) ||
-        (rc = dev_alloc(h, &h->d_st_fl, (size_t)n)))
+        (rc = dev_alloc(h, &h->d_st_kap, (size_t)n)) || (rc = dev_alloc(h, &h->d_st_fl, (size_t)n)) ||
+        (rc = dev_alloc(h, &h->d_st_list, (size_t)n)) || (rc = dev_alloc(h, &h->d_st_count, 1)))
       return rc;
   }
   StGrid g{};
@@ -1720,9 +1721,9 @@ int tbfp_surface_tension_dev(tbfp_handle *h, const double *c, double sigma, doub
   g.dyf = h->d_dyf;
   g.dyc = h->d_st_dyc;
   g.yf = h->d_st_yf;
-  launch_surface_tension(c, h->Lrho, g, 1e-12, sigma, h->d_st_cp, h->d_st_fl, h->d_st_kap, kappa, h->Lrho,
-                         (long)h->n_rho, st_x, h->Lst[0], (long)h->n_st[0], st_y, h->Lst[1], (long)h->n_st[1], st_z,
-                         h->Lst[2], (long)h->n_st[2], h->stream);
+  launch_surface_tension(c, h->Lrho, g, 1e-12, sigma, h->d_st_fl, h->d_st_kap, h->d_st_list, h->d_st_count, kappa,
+                         h->Lrho, (long)h->n_rho, h->hd_st, st_x, h->Lst[0], (long)h->n_st[0], st_y, h->Lst[1],
+                         (long)h->n_st[1], st_z, h->Lst[2], (long)h->n_st[2], h->stream);
   return finish(h, "tbfp_surface_tension");
 }
 

@@ -405,13 +405,14 @@ struct StGrid {
   double dx, dz;
   const double *dyf, *dyc, *yf;
 };
-// c: volume fraction (layout Lc); cp, fl, kap: dense scratch (c after the
-// promotion of full interface cells, class bits 1 mixed / 2 full, curvature);
-// kap_out (NULL or layout Lk, nk elements); sx, sy, sz: the three staggered
-// st arrays (nsx, nsy, nsz elements).
-void launch_surface_tension(const double *c, Lay Lc, const StGrid &g, double eps, double sigma, double *cp,
-                            unsigned char *fl, double *kap, double *kap_out, Lay Lk, long nk, double *sx, Lay Lx,
-                            long nsx, double *sy, Lay Ly, long nsy, double *sz, Lay Lz, long nsz, cudaStream_t st);
+// c: volume fraction (layout Lc); scratch fl (a class byte per cell), kap
+// (curvature, written at the mixed cells only), list (room for every cell) and
+// count (its length); kap_out (NULL or layout Lk, nk elements); sx, sy, sz: the
+// three staggered st arrays with halo hd (nsx, nsy, nsz elements).
+void launch_surface_tension(const double *c, Lay Lc, const StGrid &g, double eps, double sigma, unsigned char *fl,
+                            double *kap, int *list, int *count, double *kap_out, Lay Lk, long nk, int hd, double *sx,
+                            Lay Lx, long nsx, double *sy, Lay Ly, long nsy, double *sz, Lay Lz, long nsz,
+                            cudaStream_t st);
 
 // The all-to-all chunks of a channel split over ranks (z slabs <-> kx slabs).
 // zs[0..n]: the z-slab starts of the n ranks (zs[n] = nz of the channel).

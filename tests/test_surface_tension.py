@@ -143,3 +143,88 @@ def test_gpu_surface_tension_stretched_channel_and_projection():
         assert abs(res.max_div - ref.max_div) < 1e-12
     finally:
         eqn.close()
+
+
+def _speckled(nx, ny, nz, seed):
+    """Random volume fractions: empty, full and mixed cells side by side, so that
+    promoted cells, walls, wrapped columns and invalid directions all occur."""
+    rng = np.random.default_rng(seed)
+    c = rng.random((nz, ny, nx))
+    kind = rng.random((nz, ny, nx))
+    c[kind < 0.4] = 0.0
+    c[kind > 0.6] = 1.0
+    x = np.arange(nx)[None, None, :] + 3.0 * rng.random()
+    c[:, :, :] = np.where(np.sin(2 * np.pi * x / nx) + 0.3 * np.arange(ny)[None, :, None] / ny > 0.9, 1.0,
+                          np.where(np.sin(2 * np.pi * x / nx) < -0.8, 0.0, c))
+    return c
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n, hd_st, stretched", [((8, 4, 4), 0, False), ((12, 9, 6), 1, True), ((8, 7, 24), 3, True),
+                                                 ((96, 5, 8), 1, False), ((1024, 4, 4), 1, True)])
+def test_gpu_surface_tension_shapes(n, hd_st, stretched):
+    """Rows of one and many 32-cell chunks with and without a remainder, row
+    counts that leave a block's last warps idle, columns that wrap more than
+    once, every st halo width, an interface without and with mixed cells.  Bar:
+    the decisions are the oracle's bit for bit, the rest is rounding of a few
+    second differences of heights (1e-12 of the largest curvature)."""
+    import torch
+
+    from tbfsolver_b200.solver import FastPoissonSolver, compute_surface_tension
+
+    nx, ny, nz = n
+    g = Grid(nx, ny, nz, 2 * np.pi, 2.0, np.pi, stretched, 1.5)
+    dyf, dyc = np.ascontiguousarray(g.dyf.r(1, ny)), np.ascontiguousarray(g.dyc.r(1, ny + 1))
+    with FastPoissonSolver(g, hd_st=hd_st) as fps:
+        for c in (_speckled(nx, ny, nz, 5), np.zeros((nz, ny, nx)), np.ones((nz, ny, nx)), np.full((nz, ny, nx), 0.5)):
+            kap, *st_ref = O.surface_tension(c, 0.07, g.dx_fft, g.dz_fft, dyf, dyc)
+            f = Field("cl", 1, nx, ny, nz)
+            f.interior()[...] = c
+            cd = Field.like(f, torch.from_numpy(f.a).cuda())
+            st = VField(*[Field(k, hd_st, nx, ny, nz, torch.full(Field(k, hd_st, nx, ny, nz).a.shape, 7.0,
+                                                                dtype=torch.float64, device="cuda"))
+                          for k in ("sx", "sy", "sz")])
+            kd = Field.like(cd, torch.full_like(cd.a, 7.0))
+            torch.cuda.synchronize()
+            compute_surface_tension(fps, cd, 0.07, st, kappa=kd)
+            assert rel_linf(Field.like(kd, kd.numpy()).interior(), kap) < 1e-12
+            boxes = [(0, nx, 1, ny, 1, nz), (1, nx, 0, ny, 1, nz), (1, nx, 1, ny, 0, nz)]
+            for fd, ref, b in zip(st.components(), st_ref, boxes):
+                a = Field.like(fd, fd.numpy())
+                assert rel_linf(a.v(*b), ref) < 1e-12
+                # halos: periodic images of the interior in x and z, zero rows beyond the walls
+                lo = a.lb
+                ii = [(i - b[0]) % nx for i in range(lo[0], lo[0] + a.a.shape[2])]
+                kk = [(k - b[4]) % nz for k in range(lo[2], lo[2] + a.a.shape[0])]
+                whole = np.zeros_like(a.a)
+                j0 = b[2] - lo[1]
+                whole[:, j0:j0 + b[3] - b[2] + 1, :] = a.v(*b)[kk][:, :, ii]
+                assert np.array_equal(a.a, whole)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_gpu_surface_tension_carries_non_finite_cells(bad):
+    """A cell that is not finite makes the force of its own faces non-finite, also
+    away from every interface."""
+    import torch
+
+    from tbfsolver_b200.solver import FastPoissonSolver, compute_surface_tension
+
+    nx, ny, nz = 16, 12, 8
+    g = Grid(nx, ny, nz, 2 * np.pi, 2.0, np.pi, True, 1.5)
+    f = Field("cl", 1, nx, ny, nz)
+    if bad == np.inf:  # counts as full: among empty cells it would be promoted to a finite value
+        f.a[...] = 1.0
+    f.v(7, 7, 5, 5, 4, 4)[...] = bad
+    cd = Field.like(f, torch.from_numpy(f.a).cuda())
+    with FastPoissonSolver(g) as fps:
+        st = VField(*[Field(k, 1, nx, ny, nz, torch.zeros(Field(k, 1, nx, ny, nz).a.shape, dtype=torch.float64,
+                                                         device="cuda")) for k in ("sx", "sy", "sz")])
+        torch.cuda.synchronize()
+        compute_surface_tension(fps, cd, 0.07, st)
+        for fd, (di, dj, dk) in zip(st.components(), ((1, 0, 0), (0, 1, 0), (0, 0, 1))):
+            a = Field.like(fd, fd.numpy())
+            assert not np.isfinite(a.v(7, 7, 5, 5, 4, 4)).any()
+            assert not np.isfinite(a.v(7 - di, 7 - di, 5 - dj, 5 - dj, 4 - dk, 4 - dk)).any()
+            assert np.isnan(a.a).sum() + np.isinf(a.a).sum() == 2
