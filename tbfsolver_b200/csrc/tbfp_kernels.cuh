@@ -19,6 +19,23 @@ __host__ __device__ __forceinline__ long at(const Lay &L, int i, int j, int k) {
   return (long)(i - L.ilo) + (long)(j - L.jlo) * L.sj + (long)(k - L.klo) * L.sk;
 }
 
+// Planes per block of a kernel whose blocks march up z: the chunk size with the
+// least rounds of blocks (tiles x chunks over the blocks resident on the chip)
+// times the planes a block works through, its start-up counted as `start` of them.
+inline int march_chunk(long tiles, int planes, long slots, int start) {
+  long best = -1;
+  int kc = planes;
+  for (int n = 1; n <= planes; ++n) {
+    const int c = (planes + n - 1) / n;
+    const long cost = (tiles * ((planes + c - 1) / c) + slots - 1) / slots * (c + start);
+    if (best < 0 || cost < best) {
+      best = cost;
+      kc = c;
+    }
+  }
+  return kc;
+}
+
 // Grid constants and metric tables (device pointers, 0-based: table[j-1] holds the
 // reference's value at Fortran index j).
 struct GridK {

@@ -12,12 +12,11 @@
 // a second buffer.  Every expression follows the reference's operand order,
 // with these substitutions: a quotient by a grid spacing is a product with the
 // spacing's reciprocal (tables built once on the host, each the correctly
-// rounded 1/d); the four limiter ratios of one direction share the
-// reciprocals of their two denominators; QUICK's ratio cancels against the
-// face difference it multiplies (exact zero differences kept).  Each such term
-// differs from the reference's by an ulp or two, and the 96 FP64 divisions per
-// cell of the literal form drop to at most 22 reciprocals (4 for QUICK).  The
-// kernels are specialised per convection scheme.
+// rounded 1/d); a face value is limited on its upwind side only; the limiter's
+// ratio is multiplied out against the face difference (face_flux).  Each such
+// term differs from the reference's by an ulp or two, and the 96 FP64 divisions
+// per cell of the literal form drop to about one (1/rho), or to the faces' own
+// with van Leer's limiter.  The kernels are specialised per convection scheme.
 #include <cuda_runtime.h>
 
 #include "tbfp_kernels.cuh"
@@ -28,39 +27,6 @@ namespace {
 
 constexpr int kMT = 128;
 
-__device__ __forceinline__ double approx_zero(double d) { return d == 0.0 ? 1e-50 : d; }
-
-__device__ __forceinline__ double superbee(double r) {
-  r = fmax(0.0, r);
-  return fmax(fmax(0.0, fmin(2.0 * r, 1.0)), fmin(r, 2.0));
-}
-
-// compute_limiters (momentumEqn.f90:611-663); psi = {hpup, hpum, hmup, hmum}.
-// sharp: the localVF test of the cell (dc > epsilon(0.d0) in any direction)
-template <int S>
-__device__ __forceinline__ void limiters(double vc, double vm, double vp, double vpp, double vmm, bool sharp,
-                                         double psi[4]) {
-  if constexpr (S == 0 || S == 1) {
-    psi[0] = psi[1] = psi[2] = psi[3] = S == 0 ? 1.0 : 0.0;
-    return;
-  }
-  if (S == 5 && !sharp) {
-    psi[0] = psi[1] = psi[2] = psi[3] = 1.0;
-    return;
-  }
-  const double ip = 1.0 / approx_zero(vp - vc), im = 1.0 / approx_zero(vc - vm);
-  const double r[4] = {(vc - vm) * ip, (vpp - vp) * ip, (vm - vmm) * im, (vp - vc) * im};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const double x = r[e];
-    if constexpr (S == 2) psi[e] = (x + 3.0) * 0.25;  // (r+3)/4, exact as a product
-    else if constexpr (S == 3) {
-      const double y = fmax(0.0, x);
-      psi[e] = (y + fabs(y)) / (1.0 + fabs(y));
-    } else psi[e] = superbee(x);
-  }
-}
-
 template <int S>
 __device__ __forceinline__ bool sharp_cell(double cxp, double cxm, double cyp, double cym, double czp, double czm) {
   if constexpr (S != 5) return true;
@@ -68,66 +34,38 @@ __device__ __forceinline__ bool sharp_cell(double cxp, double cxm, double cyp, d
   return (cxp - cxm) > small || (cyp - cym) > small || (czp - czm) > small;
 }
 
-// F = max(q,0)*A + min(q,0)*B (momentumEqn.f90:247-256 and the like)
-__device__ __forceinline__ double flux(double q, double a, double b, double pu, double pm) {
-  const double A = a + 0.5 * pu * (b - a);
-  const double B = b + 0.5 * pm * (a - b);
-  return fmax(q, 0.0) * A + fmin(q, 0.0) * B;
-}
-
-// Fp - Fm of one direction: the limited flux through the upper face (between
-// vc and vp) minus the one through the lower face (between vm and vc)
-// (momentumEqn.f90:240-256 and the like).  QUICK's limiter is psi = (r+3)/4
-// with r a ratio whose denominator is the face's own difference d, so the
-// flux's psi*d/2 is ((numerator) + 3d)/8 without the division; d == 0 keeps
-// the reference's value (approx_zero makes psi*d exactly 0 there).
-template <int S>
-__device__ __forceinline__ double conv_diff(double qp, double qm, double vmm, double vm, double vc, double vp,
-                                            double vpp, bool sh) {
-  if constexpr (S == 2) {
-    const double d = vp - vc, e = vc - vm;
-    const double Ap = d == 0.0 ? vc : vc + 0.125 * (e + 3.0 * d);
-    const double Bp = d == 0.0 ? vp : vp - 0.125 * ((vpp - vp) + 3.0 * d);
-    const double Am = e == 0.0 ? vm : vm + 0.125 * ((vm - vmm) + 3.0 * e);
-    const double Bm = e == 0.0 ? vc : vc - 0.125 * (d + 3.0 * e);
-    return (fmax(qp, 0.0) * Ap + fmin(qp, 0.0) * Bp) - (fmax(qm, 0.0) * Am + fmin(qm, 0.0) * Bm);
-  } else {
-    double ps[4];
-    limiters<S>(vc, vm, vp, vpp, vmm, sh, ps);
-    return flux(qp, vc, vp, ps[0], ps[1]) - flux(qm, vm, vc, ps[2], ps[3]);
-  }
-}
-
-// the limiter of one ratio (momentumEqn.f90:667-734) for schemes 3 and 4
-template <int S>
-__device__ __forceinline__ double lim(double x) {
-  if constexpr (S == 3) {
-    const double y = fmax(0.0, x);
-    return (y + fabs(y)) / (1.0 + fabs(y));
-  } else {
-    return superbee(x);
-  }
-}
-
 // The limited flux through the face between vc and vp (vm and vpp the next
-// values outward), for schemes 0-4, whose limiters depend on the face alone:
-// the upper face of one cell is then the lower face of the next bit for bit
-// (the lower face's ratios have the same numerators and denominator), so a
-// face is computed once.
+// values outward): max(q,0)*A + min(q,0)*B with A = vc + psi(r)/2 (vp - vc),
+// r = (vc - vm)/(vp - vc), and B its mirror image (momentumEqn.f90:240-256 and
+// the like; limiters :611-734).  One of the products is always zero, so only
+// the upwind side is evaluated: a the upwind value, f the one behind it, d the
+// difference across the face, n = a - f, r = n/d.  (An infinity or NaN on the
+// other side's far value then stays out of this face; it is in the face beside
+// it.)  psi(r) d is written without the ratio:
+//   QUICK     (r+3)/4 d            = (n + 3d)/4, and 0 for d = 0 (the reference's
+//                                    approx_zero makes it so)
+//   van Leer  (r+|r|)/(1+|r|) d    = 2 n d/(n + d) for n, d of one sign, else 0
+//   superbee  max(0, min(2r,1), min(r,2)) d = min(2 min(|n|,|d|), max(|n|,|d|))
+//                                    with d's sign for n, d of one sign, else 0
+// sh: scheme 5's test of the cell (superbee where the volume fraction varies,
+// central elsewhere); the other schemes depend on the face alone, so the upper
+// face of one cell is the lower face of the next, bit for bit: the last product
+// is not contracted into what the flux is used in.
 template <int S>
-__device__ __forceinline__ double face_flux(double q, double vm, double vc, double vp, double vpp) {
-  if constexpr (S == 2) {
-    const double d = vp - vc;
-    const double A = d == 0.0 ? vc : vc + 0.125 * ((vc - vm) + 3.0 * d);
-    const double B = d == 0.0 ? vp : vp - 0.125 * ((vpp - vp) + 3.0 * d);
-    return fmax(q, 0.0) * A + fmin(q, 0.0) * B;
-  } else if constexpr (S == 0 || S == 1) {
-    const double p = S == 0 ? 1.0 : 0.0;
-    return flux(q, vc, vp, p, p);
-  } else {
-    const double ip = 1.0 / approx_zero(vp - vc);
-    return flux(q, vc, vp, lim<S>((vc - vm) * ip), lim<S>((vpp - vp) * ip));
-  }
+__device__ __forceinline__ double face_flux(double q, double vm, double vc, double vp, double vpp, bool sh) {
+  const bool up = q > 0.0;
+  const double a = up ? vc : vp;
+  if constexpr (S == 1) return __dmul_rn(q, a);
+  const double d = (up ? vp : vc) - a;
+  if (S == 0 || (S == 5 && !sh)) return __dmul_rn(q, a + 0.5 * d);
+  const double n = a - (up ? vm : vpp);
+  if constexpr (S == 2) return __dmul_rn(q, d == 0.0 ? a : a + 0.125 * (n + 3.0 * d));
+  const bool same = n * d > 0.0;
+  if constexpr (S == 3) return __dmul_rn(q, same ? a + n * (d / (n + d)) : a);
+  const double an = fabs(n), ad = fabs(d);
+  const double lo = an < ad ? an : ad, hi = an < ad ? ad : an;
+  const double m = 2.0 * lo < hi ? lo : 0.5 * hi;  // half of |psi(r) d|
+  return __dmul_rn(q, same ? a + copysign(m, d) : a);
 }
 
 struct MomArgs {
@@ -138,6 +76,7 @@ struct MomArgs {
   double *phx, *phy, *phz;  // fluxes, dense over the equation boxes
   int nx, ny, nz;
   int hdu, hdc;  // halos of the velocity and cell arrays
+  int kc;        // planes per block of the tiled kernel
   // the out-of-place form's update (addConvDiff + addSource) into uxo, uyo, uzo
   double *uxo, *uyo, *uzo;
   const double *ppx, *ppy, *ppz, *stx, *sty, *stz;
@@ -145,54 +84,54 @@ struct MomArgs {
   double dt, gamma, xi, r, invrho0, fs, gch, g;
 };
 
-// one component's flux into its buffer and, in the out-of-place form, its
+
+// element offsets; every array holds fewer than 2^31 elements (checked at set-up)
+__device__ __forceinline__ int box_x(const MomArgs &a, int i, int j, int k) {
+  return ((k - 1) * a.ny + (j - 1)) * (a.nx + 1) + i;
+}
+__device__ __forceinline__ int box_y(const MomArgs &a, int i, int j, int k) {
+  return ((k - 1) * (a.ny - 1) + (j - 1)) * a.nx + (i - 1);
+}
+__device__ __forceinline__ int box_z(const MomArgs &a, int i, int j, int k) {
+  return (k * a.ny + (j - 1)) * a.nx + (i - 1);
+}
+__device__ __forceinline__ int at32(const Lay &L, int i, int j, int k) {
+  return (i - L.ilo) + (j - L.jlo) * (int)L.sj + (k - L.klo) * (int)L.sk;
+}
+
+// One component's flux into its buffer and, in the out-of-place form, its
 // addConvDiff + addSource update from the thread's own u (the expressions of
-// k_momentum_update, so both forms give the same values)
+// k_momentum_update, so both forms give the same values).  pp: the last step's
+// flux, loaded by the caller well before.
 template <bool OUT>
-__device__ __forceinline__ void emit_x(const MomArgs &a, int i, int j, int k, double phi, double uc, double invrho);
-template <bool OUT>
-__device__ __forceinline__ void emit_y(const MomArgs &a, int i, int j, int k, double phi, double uc);
-template <bool OUT>
-__device__ __forceinline__ void emit_z(const MomArgs &a, int i, int j, int k, double phi, double uc);
-
-__device__ __forceinline__ long box_x(const MomArgs &a, int i, int j, int k) {
-  return ((long)(k - 1) * a.ny + (j - 1)) * (a.nx + 1) + i;
-}
-__device__ __forceinline__ long box_y(const MomArgs &a, int i, int j, int k) {
-  return ((long)(k - 1) * (a.ny - 1) + (j - 1)) * a.nx + (i - 1);
-}
-__device__ __forceinline__ long box_z(const MomArgs &a, int i, int j, int k) {
-  return ((long)k * a.ny + (j - 1)) * a.nx + (i - 1);
-}
-
-template <bool OUT>
-__device__ __forceinline__ void emit_x(const MomArgs &a, int i, int j, int k, double phi, double uc, double invrho) {
-  const long q = box_x(a, i, j, k);
+__device__ __forceinline__ void emit_x(const MomArgs &a, int i, int j, int k, double phi, double uc, double invrho,
+                                       double pp) {
+  const int q = box_x(a, i, j, k);
   a.phx[q] = phi;
   if constexpr (OUT) {
-    const double u = uc + a.dt * (a.gamma * phi + a.xi * __ldg(a.ppx + q));
-    const double st = a.stx ? __ldg(a.stx + at(a.Lsx, i, j, k)) : 0.0;
-    a.uxo[at(a.Lux, i, j, k)] = u + a.invrho0 * a.r * st + invrho * a.r * a.fs + a.r * a.gch;
+    const double u = uc + a.dt * (a.gamma * phi + a.xi * pp);
+    const double st = a.stx ? __ldg(a.stx + at32(a.Lsx, i, j, k)) : 0.0;
+    a.uxo[at32(a.Lux, i, j, k)] = u + a.invrho0 * a.r * st + invrho * a.r * a.fs + a.r * a.gch;
   }
 }
 template <bool OUT>
-__device__ __forceinline__ void emit_y(const MomArgs &a, int i, int j, int k, double phi, double uc) {
-  const long q = box_y(a, i, j, k);
+__device__ __forceinline__ void emit_y(const MomArgs &a, int i, int j, int k, double phi, double uc, double pp) {
+  const int q = box_y(a, i, j, k);
   a.phy[q] = phi;
   if constexpr (OUT) {
-    const double u = uc + a.dt * (a.gamma * phi + a.xi * __ldg(a.ppy + q));
-    const double st = a.sty ? __ldg(a.sty + at(a.Lsy, i, j, k)) : 0.0;
-    a.uyo[at(a.Luy, i, j, k)] = u + a.invrho0 * a.r * st + a.r * a.g;
+    const double u = uc + a.dt * (a.gamma * phi + a.xi * pp);
+    const double st = a.sty ? __ldg(a.sty + at32(a.Lsy, i, j, k)) : 0.0;
+    a.uyo[at32(a.Luy, i, j, k)] = u + a.invrho0 * a.r * st + a.r * a.g;
   }
 }
 template <bool OUT>
-__device__ __forceinline__ void emit_z(const MomArgs &a, int i, int j, int k, double phi, double uc) {
-  const long q = box_z(a, i, j, k);
+__device__ __forceinline__ void emit_z(const MomArgs &a, int i, int j, int k, double phi, double uc, double pp) {
+  const int q = box_z(a, i, j, k);
   a.phz[q] = phi;
   if constexpr (OUT) {
-    const double u = uc + a.dt * (a.gamma * phi + a.xi * __ldg(a.ppz + q));
-    const double st = a.stz ? __ldg(a.stz + at(a.Lsz, i, j, k)) : 0.0;
-    a.uzo[at(a.Luz, i, j, k)] = u + a.invrho0 * a.r * st;
+    const double u = uc + a.dt * (a.gamma * phi + a.xi * pp);
+    const double st = a.stz ? __ldg(a.stz + at32(a.Lsz, i, j, k)) : 0.0;
+    a.uzo[at32(a.Luz, i, j, k)] = u + a.invrho0 * a.r * st;
   }
 }
 
@@ -221,16 +160,33 @@ struct GAcc {
   __device__ double c(int di, int dj, int dk) const { return __ldg(pC + (di + dj * cj + dk * ck)); }
   __device__ double m(int di, int dj, int dk) const { return __ldg(pM + (di + dj * cj + dk * ck)); }
   __device__ double r(int di, int dj, int dk) const { return __ldg(pR + (di + dj * cj + dk * ck)); }
+  __device__ GAcc shifted(int di, int dj) const {
+    GAcc b = *this;
+    b.pU += di + dj * uj;
+    b.pV += di + dj * vj;
+    b.pW += di + dj * wj;
+    return b;
+  }
+  __device__ GAcc down() const {
+    GAcc b = *this;
+    b.pU -= uk;
+    b.pV -= vk;
+    b.pW -= wk;
+    return b;
+  }
 };
 
 // tiled kernel geometry: a 32 x 8 tile of (i, j) columns marches up in k; the
 // velocity planes k-2..k+2 (in-plane halo 2) and the cell planes k-1..k+1
 // (halo 1) sit in rings of shared memory, the next plane loading meanwhile
-constexpr int kTX = 32, kTY = 8, kKC = 64;
+constexpr int kTX = 32, kTY = 8;
 constexpr int kHV = 2, kHC = 1;
 constexpr int kPV = kTX + 2 * kHV, kPC = kTX + 2 * kHC;  // row pitches
 constexpr int kNV = kPV * (kTY + 2 * kHV), kNC = kPC * (kTY + 2 * kHC);  // doubles per plane
-constexpr int kRV = 6, kRC = 4;  // ring depths: 5 + 1 and 3 + 1 planes
+constexpr int kRC = 4;  // ring depth of the cell planes: 3 + 1 arriving
+// and of the velocity planes: k-1..k+2 + 1 arriving; scheme 5 also reads k-2 in
+// every step (its lower z faces are not carried)
+__host__ __device__ constexpr int ring_v(int S) { return S == 5 ? 6 : 5; }
 
 struct SAcc {
   const double *sU, *sV, *sW, *sC, *sM, *sR;
@@ -241,24 +197,20 @@ struct SAcc {
   __device__ double c(int di, int dj, int dk) const { return sC[oc[dk + 1] + dj * kPC + di]; }
   __device__ double m(int di, int dj, int dk) const { return sM[oc[dk + 1] + dj * kPC + di]; }
   __device__ double r(int di, int dj, int dk) const { return sR[oc[dk + 1] + dj * kPC + di]; }
-  // the accessor of the cell (di, dj) columns away in the same plane
+  // the accessor of the cell (di, dj) columns away in the same plane, for the velocities
   __device__ SAcc shifted(int di, int dj) const {
     SAcc b = *this;
     b.sU += di + dj * kPV;
     b.sV += di + dj * kPV;
     b.sW += di + dj * kPV;
-    b.sC += di + dj * kPC;
-    b.sM += di + dj * kPC;
-    b.sR += di + dj * kPC;
     return b;
   }
-  // the accessor of the cell one plane down (reaches planes k-2..k+1 only)
+  // the accessor of the cell one plane down, for the velocities (reaches planes k-2..k+1 only;
+  // with five planes in the ring k-2 is there in the chunk's first step only)
   __device__ SAcc down() const {
     SAcc b = *this;
 #pragma unroll
     for (int d = 4; d > 0; --d) b.ov[d] = ov[d - 1];
-#pragma unroll
-    for (int d = 2; d > 0; --d) b.oc[d] = oc[d - 1];
     return b;
   }
 };
@@ -286,53 +238,53 @@ struct Met {
 // The upper-face fluxes of the nine (component, direction) pairs at the
 // accessor's cell (updateConveDiff, momentumEqn.f90:228-603): ux faces
 template <int S, class Acc>
-__device__ __forceinline__ double F_xx(const Acc &A) {
+__device__ __forceinline__ double F_xx(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (u(0, 0, 0) + u(1, 0, 0)), u(-1, 0, 0), u(0, 0, 0), u(1, 0, 0), u(2, 0, 0));
+  return face_flux<S>(0.5 * (u(0, 0, 0) + u(1, 0, 0)), u(-1, 0, 0), u(0, 0, 0), u(1, 0, 0), u(2, 0, 0), sh);
 }
 template <int S, class Acc>
-__device__ __forceinline__ double F_xy(const Acc &A) {
+__device__ __forceinline__ double F_xy(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (v(1, 0, 0) + v(0, 0, 0)), u(0, -1, 0), u(0, 0, 0), u(0, 1, 0), u(0, 2, 0));
+  return face_flux<S>(0.5 * (v(1, 0, 0) + v(0, 0, 0)), u(0, -1, 0), u(0, 0, 0), u(0, 1, 0), u(0, 2, 0), sh);
 }
 template <int S, class Acc>
-__device__ __forceinline__ double F_xz(const Acc &A) {
+__device__ __forceinline__ double F_xz(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (w(0, 0, 0) + w(1, 0, 0)), u(0, 0, -1), u(0, 0, 0), u(0, 0, 1), u(0, 0, 2));
+  return face_flux<S>(0.5 * (w(0, 0, 0) + w(1, 0, 0)), u(0, 0, -1), u(0, 0, 0), u(0, 0, 1), u(0, 0, 2), sh);
 }
 // uy faces
 template <int S, class Acc>
-__device__ __forceinline__ double F_yx(const Acc &A, const Met &g) {
+__device__ __forceinline__ double F_yx(const Acc &A, const Met &g, bool sh = true) {
   TBFP_MOM_ACCESSORS;
   return face_flux<S>(0.5 * (u(0, 1, 0) * g.dyf1 + u(0, 0, 0) * g.dyf0) * g.ryc1, v(-1, 0, 0), v(0, 0, 0), v(1, 0, 0),
-                      v(2, 0, 0));
+                      v(2, 0, 0), sh);
 }
 template <int S, class Acc>
-__device__ __forceinline__ double F_yy(const Acc &A) {
+__device__ __forceinline__ double F_yy(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (v(0, 0, 0) + v(0, 1, 0)), v(0, -1, 0), v(0, 0, 0), v(0, 1, 0), v(0, 2, 0));
+  return face_flux<S>(0.5 * (v(0, 0, 0) + v(0, 1, 0)), v(0, -1, 0), v(0, 0, 0), v(0, 1, 0), v(0, 2, 0), sh);
 }
 template <int S, class Acc>
-__device__ __forceinline__ double F_yz(const Acc &A, const Met &g) {
+__device__ __forceinline__ double F_yz(const Acc &A, const Met &g, bool sh = true) {
   TBFP_MOM_ACCESSORS;
   return face_flux<S>(0.5 * (w(0, 1, 0) * g.dyf1 + w(0, 0, 0) * g.dyf0) * g.ryc1, v(0, 0, -1), v(0, 0, 0), v(0, 0, 1),
-                      v(0, 0, 2));
+                      v(0, 0, 2), sh);
 }
 // uz faces
 template <int S, class Acc>
-__device__ __forceinline__ double F_zx(const Acc &A) {
+__device__ __forceinline__ double F_zx(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (u(0, 0, 0) + u(0, 0, 1)), w(-1, 0, 0), w(0, 0, 0), w(1, 0, 0), w(2, 0, 0));
+  return face_flux<S>(0.5 * (u(0, 0, 0) + u(0, 0, 1)), w(-1, 0, 0), w(0, 0, 0), w(1, 0, 0), w(2, 0, 0), sh);
 }
 template <int S, class Acc>
-__device__ __forceinline__ double F_zy(const Acc &A) {
+__device__ __forceinline__ double F_zy(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (v(0, 0, 0) + v(0, 0, 1)), w(0, -1, 0), w(0, 0, 0), w(0, 1, 0), w(0, 2, 0));
+  return face_flux<S>(0.5 * (v(0, 0, 0) + v(0, 0, 1)), w(0, -1, 0), w(0, 0, 0), w(0, 1, 0), w(0, 2, 0), sh);
 }
 template <int S, class Acc>
-__device__ __forceinline__ double F_zz(const Acc &A) {
+__device__ __forceinline__ double F_zz(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (w(0, 0, 0) + w(0, 0, 1)), w(0, 0, -1), w(0, 0, 0), w(0, 0, 1), w(0, 0, 2));
+  return face_flux<S>(0.5 * (w(0, 0, 0) + w(0, 0, 1)), w(0, 0, -1), w(0, 0, 0), w(0, 0, 1), w(0, 0, 2), sh);
 }
 
 // x component at face (i, j, k) (momentumEqn.f90:228-341) from the convective
@@ -411,111 +363,138 @@ __device__ __forceinline__ double tail_z(const Acc &A, const Met &g, double invr
   return phi + (dxx + dyy + dzz + dxxt + dyyt + dzzt) * invrho;
 }
 
-// The per-cell forms (every scheme; scheme 5's limiters depend on the cell):
-// both faces of each direction at the cell itself
-template <int S, class Acc>
-__device__ __forceinline__ double phi_x(const Acc &A, const Met &g, double invrho) {
+// The per-cell forms: both x and y faces of each component at the cell itself;
+// the z flux differences (cz) are formed by the caller, except for scheme 5,
+// whose limiters depend on the cell (Z: form them here).
+template <int S, bool Z, class Acc>
+__device__ __forceinline__ double phi_x(const Acc &A, const Met &g, double invrho, double cz) {
   TBFP_MOM_ACCESSORS;
   const bool sh = sharp_cell<S>(c(1, 0, 0), c(0, 0, 0), c(0, 1, 0), c(0, -1, 0), c(0, 0, 1), c(0, 0, -1));
-  const double uc = u(0, 0, 0);
-  const double cx = conv_diff<S>(0.5 * (uc + u(1, 0, 0)), 0.5 * (uc + u(-1, 0, 0)), u(-2, 0, 0), u(-1, 0, 0), uc,
-                                 u(1, 0, 0), u(2, 0, 0), sh);
-  const double cy = conv_diff<S>(0.5 * (v(1, 0, 0) + v(0, 0, 0)), 0.5 * (v(1, -1, 0) + v(0, -1, 0)), u(0, -2, 0),
-                                 u(0, -1, 0), uc, u(0, 1, 0), u(0, 2, 0), sh);
-  const double cz = conv_diff<S>(0.5 * (w(0, 0, 0) + w(1, 0, 0)), 0.5 * (w(0, 0, -1) + w(1, 0, -1)), u(0, 0, -2),
-                                 u(0, 0, -1), uc, u(0, 0, 1), u(0, 0, 2), sh);
+  const double cx = F_xx<S>(A, sh) - F_xx<S>(A.shifted(-1, 0), sh);
+  const double cy = F_xy<S>(A, sh) - F_xy<S>(A.shifted(0, -1), sh);
+  if constexpr (Z) cz = F_xz<S>(A, sh) - F_xz<S>(A.down(), sh);
   return tail_x(A, g, invrho, cx, cy, cz);
 }
 
-template <int S, class Acc>
-__device__ __forceinline__ double phi_y(const Acc &A, const Met &g, double invrho) {
+template <int S, bool Z, class Acc>
+__device__ __forceinline__ double phi_y(const Acc &A, const Met &g, double invrho, double cz) {
   TBFP_MOM_ACCESSORS;
   const bool sh = sharp_cell<S>(c(1, 0, 0), c(-1, 0, 0), c(0, 1, 0), c(0, 0, 0), c(0, 0, 1), c(0, 0, -1));
-  const double vc = v(0, 0, 0);
-  const double dyfj = g.dyf0, dyfp = g.dyf1, rycp = g.ryc1;
-  const double cx = conv_diff<S>(0.5 * (u(0, 1, 0) * dyfp + u(0, 0, 0) * dyfj) * rycp,
-                                 0.5 * (u(-1, 1, 0) * dyfp + u(-1, 0, 0) * dyfj) * rycp, v(-2, 0, 0), v(-1, 0, 0), vc,
-                                 v(1, 0, 0), v(2, 0, 0), sh);
-  const double cy = conv_diff<S>(0.5 * (vc + v(0, 1, 0)), 0.5 * (vc + v(0, -1, 0)), v(0, -2, 0), v(0, -1, 0), vc,
-                                 v(0, 1, 0), v(0, 2, 0), sh);
-  const double cz = conv_diff<S>(0.5 * (w(0, 1, 0) * dyfp + w(0, 0, 0) * dyfj) * rycp,
-                                 0.5 * (w(0, 1, -1) * dyfp + w(0, 0, -1) * dyfj) * rycp, v(0, 0, -2), v(0, 0, -1), vc,
-                                 v(0, 0, 1), v(0, 0, 2), sh);
+  const double cx = F_yx<S>(A, g, sh) - F_yx<S>(A.shifted(-1, 0), g, sh);
+  const double cy = F_yy<S>(A, sh) - F_yy<S>(A.shifted(0, -1), sh);
+  if constexpr (Z) cz = F_yz<S>(A, g, sh) - F_yz<S>(A.down(), g, sh);
   return tail_y(A, g, invrho, cx, cy, cz);
 }
 
-template <int S, class Acc>
-__device__ __forceinline__ double phi_z(const Acc &A, const Met &g, double invrho) {
+template <int S, bool Z, class Acc>
+__device__ __forceinline__ double phi_z(const Acc &A, const Met &g, double invrho, double cz) {
   TBFP_MOM_ACCESSORS;
   const bool sh = sharp_cell<S>(c(1, 0, 0), c(-1, 0, 0), c(0, 1, 0), c(0, -1, 0), c(0, 0, 1), c(0, 0, 0));
-  const double wc = w(0, 0, 0);
-  const double cx = conv_diff<S>(0.5 * (u(0, 0, 0) + u(0, 0, 1)), 0.5 * (u(-1, 0, 0) + u(-1, 0, 1)), w(-2, 0, 0),
-                                 w(-1, 0, 0), wc, w(1, 0, 0), w(2, 0, 0), sh);
-  const double cy = conv_diff<S>(0.5 * (v(0, 0, 0) + v(0, 0, 1)), 0.5 * (v(0, -1, 0) + v(0, -1, 1)), w(0, -2, 0),
-                                 w(0, -1, 0), wc, w(0, 1, 0), w(0, 2, 0), sh);
-  const double cz = conv_diff<S>(0.5 * (wc + w(0, 0, 1)), 0.5 * (wc + w(0, 0, -1)), w(0, 0, -2), w(0, 0, -1), wc,
-                                 w(0, 0, 1), w(0, 0, 2), sh);
+  const double cx = F_zx<S>(A, sh) - F_zx<S>(A.shifted(-1, 0), sh);
+  const double cy = F_zy<S>(A, sh) - F_zy<S>(A.shifted(0, -1), sh);
+  if constexpr (Z) cz = F_zz<S>(A, sh) - F_zz<S>(A.down(), sh);
   return tail_z(A, g, invrho, cx, cy, cz);
 }
 #undef TBFP_MOM_ACCESSORS
 
-// Computing each face once (schemes 0-4) costs a barrier, shared-memory
-// traffic and the edge faces; it pays where the limiter is expensive (van
-// Leer's and superbee's divisions and branches: 27 % and 22 % faster on
-// 512x384x256) and loses where it is cheap (central, upwind, QUICK: 8-10 %
-// slower), so those keep both faces per cell, as scheme 5 must.
-__host__ __device__ constexpr bool share_faces(int S) { return S == 3 || S == 4; }
+constexpr int kMomBlocks = 2;  // blocks per SM
 
 // Tiled form: block (32, 8) over a tile of (i, j) columns, i = 1..nx,
-// j = 1..ny, marching k over a chunk of kKC planes of 0..nz; each thread the
+// j = 1..ny, marching k over a chunk of a.kc planes of 0..nz; each thread the
 // components whose box holds its (i, j, k).  A plane outside a field's array
 // is not loaded: no stencil of a computed component reaches it.
+// The rho ring holds 1/rho: a plane is inverted in place, once per element, in
+// the step before the one that computes on it.
+// Bound: FP64 latency and instructions at 16 warps per SM (registers and the
+// plane rings allow two blocks).  512x384x256, out of place, by scheme 0..5:
+// 2.25 2.17 2.32 3.48 2.68 3.02 ms, where limiters evaluated on both sides of each
+// face, three reciprocals of rho per cell, the last step's fluxes loaded where
+// they are used, and lower z faces evaluated again took 3.06 3.07 3.29 8.97 5.21
+// 4.15 ms.  Three blocks per SM (80 registers) spill: 3.76 ms for QUICK.  Each x
+// and y face computed once per tile (shared memory and a barrier) does not pay
+// any more: 3.68 against 3.56 ms for van Leer's limiter, the dearest.
 template <int S, bool OUT>
-__global__ void __launch_bounds__(kTX * kTY, 2) k_momentum_fluxes(MomArgs a) {
+__global__ void __launch_bounds__(kTX * kTY, kMomBlocks) k_momentum_fluxes(MomArgs a) {
   extern __shared__ double sm[];
+  constexpr int kRV = ring_v(S);
   double *rU = sm, *rV = rU + kRV * kNV, *rW = rV + kRV * kNV;
   double *rM = rW + kRV * kNV, *rR = rM + kRC * kNC, *rC = rR + kRC * kNC;
-  // face fluxes of one plane (schemes 0-4): x faces [3][kTY][kTX+1], y faces [3][kTY+1][kTX]
-  double *fx = rC, *fy = fx + 3 * kTY * (kTX + 1);
   double fzl0 = 0.0, fzl1 = 0.0, fzl2 = 0.0;  // lower z faces of the current plane
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTX + tx;
   const int i0 = blockIdx.x * kTX + 1, j0 = blockIdx.y * kTY + 1;
-  const int kb = blockIdx.z * kKC, ke = min(kb + kKC - 1, a.nz);
+  const int kb = blockIdx.z * a.kc, ke = min(kb + a.kc - 1, a.nz);
   const int i = i0 + tx, j = j0 + ty;
   const bool in = i <= a.nx && j <= a.ny;
   const int vhi = a.hdu, chi = a.hdc;  // upper bound of every array: n + halo
 
-  auto load_v = [&](double *ring, const double *f, const Lay &L, int kp) {
+  // The thread's elements of a plane: ring offsets tid + 256 e, and their
+  // offsets in the arrays' planes (-1: outside the array), the same for every k.
+  constexpr int kT = kTX * kTY, kEV = (kNV + kT - 1) / kT, kEC = (kNC + kT - 1) / kT;
+  int gU[kEV], gV[kEV], gW[kEV], gC[kEC];
+#pragma unroll
+  for (int e = 0; e < kEV; ++e) {
+    const int o = tid + kT * e, rr = o / kPV, gi = i0 - kHV + (o - rr * kPV), gj = j0 - kHV + rr;
+    auto off = [&](const Lay &L) {
+      const bool ok = o < kNV && gi >= L.ilo && gi <= a.nx + vhi && gj >= L.jlo && gj <= a.ny + vhi;
+      return ok ? at32(L, gi, gj, L.klo) : -1;
+    };
+    gU[e] = off(a.Lux);
+    gV[e] = off(a.Luy);
+    gW[e] = off(a.Luz);
+  }
+#pragma unroll
+  for (int e = 0; e < kEC; ++e) {
+    const int o = tid + kT * e, rr = o / kPC, gi = i0 - kHC + (o - rr * kPC), gj = j0 - kHC + rr;
+    const bool ok = o < kNC && gi >= a.Lc.ilo && gi <= a.nx + chi && gj >= a.Lc.jlo && gj <= a.ny + chi;
+    gC[e] = ok ? at32(a.Lc, gi, gj, a.Lc.klo) : -1;
+  }
+  auto load_v = [&](double *ring, const double *f, const Lay &L, const int(&g)[kEV], int kp) {
     if (kp < L.klo || kp > a.nz + vhi) return;
-    double *dst = ring + ((kp + 3 * kRV) % kRV) * kNV;
-    for (int e = tid; e < kNV; e += kTX * kTY) {
-      const int rr = e / kPV, cc = e - rr * kPV;
-      const int gi = i0 - kHV + cc, gj = j0 - kHV + rr;
-      if (gi >= L.ilo && gi <= a.nx + vhi && gj >= L.jlo && gj <= a.ny + vhi) cp_async8(dst + e, f + at(L, gi, gj, kp));
-    }
+    double *dst = ring + ((kp + 3 * kRV) % kRV) * kNV + tid;
+    const double *src = f + (kp - L.klo) * L.sk;
+#pragma unroll
+    for (int e = 0; e < kEV; ++e)
+      if (g[e] >= 0) cp_async8(dst + kT * e, src + g[e]);
   };
   auto load_c = [&](double *ring, const double *f, int kp) {
-    const Lay &L = a.Lc;
-    if (kp < L.klo || kp > a.nz + chi) return;
-    double *dst = ring + ((kp + 3 * kRC) % kRC) * kNC;
-    for (int e = tid; e < kNC; e += kTX * kTY) {
-      const int rr = e / kPC, cc = e - rr * kPC;
-      const int gi = i0 - kHC + cc, gj = j0 - kHC + rr;
-      if (gi >= L.ilo && gi <= a.nx + chi && gj >= L.jlo && gj <= a.ny + chi) cp_async8(dst + e, f + at(L, gi, gj, kp));
-    }
+    if (kp < a.Lc.klo || kp > a.nz + chi) return;
+    double *dst = ring + ((kp + 3 * kRC) % kRC) * kNC + tid;
+    const double *src = f + (kp - a.Lc.klo) * a.Lc.sk;
+#pragma unroll
+    for (int e = 0; e < kEC; ++e)
+      if (gC[e] >= 0) cp_async8(dst + kT * e, src + gC[e]);
   };
   auto load_planes = [&](int kv, int kcl) {
-    load_v(rU, a.ux, a.Lux, kv);
-    load_v(rV, a.uy, a.Luy, kv);
-    load_v(rW, a.uz, a.Luz, kv);
+    load_v(rU, a.ux, a.Lux, gU, kv);
+    load_v(rV, a.uy, a.Luy, gV, kv);
+    load_v(rW, a.uz, a.Luz, gW, kv);
     load_c(rM, a.mu, kcl);
     load_c(rR, a.rho, kcl);
     if (S == 5) load_c(rC, a.c, kcl);
   };
+  // 1/rho of plane kp in place: the thread's own element (read by the thread
+  // itself one plane below, before the barrier), and the columns i0 + 32 and
+  // rows j0 + 8 that only neighbours read, by the threads of the first rows
+  auto invert = [&](int kp) {
+    double *pl = rR + ((kp + 3 * kRC) % kRC) * kNC;
+    if (in) {
+      double *own = pl + (ty + kHC) * kPC + tx + kHC;
+      *own = 1.0 / *own;
+    }
+    if (ty == 0 && i <= a.nx && j0 + kTY <= a.ny) {
+      double *row = pl + (kTY + kHC) * kPC + tx + kHC;
+      *row = 1.0 / *row;
+    }
+    // the column right of the tile, or of the grid's last column
+    if (ty == 1 && tx < kTY && j0 + tx <= a.ny) {
+      double *col = pl + (tx + kHC) * kPC + min(kTX, a.nx + 1 - i0) + kHC;
+      *col = 1.0 / *col;
+    }
+  };
   for (int d = -2; d <= 2; ++d) {
-    load_v(rU, a.ux, a.Lux, kb + d);
-    load_v(rV, a.uy, a.Luy, kb + d);
-    load_v(rW, a.uz, a.Luz, kb + d);
+    load_v(rU, a.ux, a.Lux, gU, kb + d);
+    load_v(rV, a.uy, a.Luy, gV, kb + d);
+    load_v(rW, a.uz, a.Luz, gW, kb + d);
   }
   for (int d = -1; d <= 1; ++d) {
     load_c(rM, a.mu, kb + d);
@@ -524,6 +503,8 @@ __global__ void __launch_bounds__(kTX * kTY, 2) k_momentum_fluxes(MomArgs a) {
   }
   cp_async_wait_all();
   __syncthreads();
+  invert(kb);
+  __syncthreads();
   SAcc A;
   A.sU = rU + (ty + kHV) * kPV + tx + kHV;
   A.sV = rV + (ty + kHV) * kPV + tx + kHV;
@@ -531,89 +512,69 @@ __global__ void __launch_bounds__(kTX * kTY, 2) k_momentum_fluxes(MomArgs a) {
   A.sM = rM + (ty + kHC) * kPC + tx + kHC;
   A.sR = rR + (ty + kHC) * kPC + tx + kHC;
   A.sC = rC + (ty + kHC) * kPC + tx + kHC;
-  for (int k = kb; k <= ke; ++k) {
-    // planes k+3 (velocity) and k+2 (cell) into the slots of k-3 and k-2, read by the previous step only
-    if (k < ke) load_planes(k + 3, k + 2);
+  auto at_plane = [&](int k) {
 #pragma unroll
     for (int d = 0; d < 5; ++d) A.ov[d] = ((k + d - 2 + 3 * kRV) % kRV) * kNV;
 #pragma unroll
     for (int d = 0; d < 3; ++d) A.oc[d] = ((k + d - 1 + 3 * kRC) % kRC) * kNC;
-    if constexpr (!share_faces(S)) {
-      if (in) {
-        const double irc = 1.0 / A.r(0, 0, 0);  // 1/rho of the own cell, shared by the three components
-        const Met g(a, i, j, k);
-        if (k >= 1) {
-          const double ivx = 0.5 * (1.0 / A.r(1, 0, 0) + irc);
-          emit_x<OUT>(a, i, j, k, phi_x<S>(A, g, ivx), A.u(0, 0, 0), ivx);
-          if (j <= a.ny - 1) emit_y<OUT>(a, i, j, k, phi_y<S>(A, g, 0.5 * (1.0 / A.r(0, 1, 0) + irc)), A.v(0, 0, 0));
-        }
-        emit_z<OUT>(a, i, j, k, phi_z<S>(A, g, 0.5 * (1.0 / A.r(0, 0, 1) + irc)), A.w(0, 0, 0));
+  };
+  if constexpr (S != 5) {  // the chunk's first lower z faces (ux, uy need none at k = 0)
+    if (in) {
+      at_plane(kb);
+      const SAcc B = A.down();
+      if (kb > 0) {
+        fzl0 = F_xz<S>(B);
+        fzl1 = F_yz<S>(B, Met(a, i, j, kb));
       }
-    } else {
-      // each face once: the cell's upper x, y faces into shared memory, its
-      // upper z faces in registers (the next plane's lower ones); the tile's
-      // lower edge faces by warp 0 (x, 8 rows) and warp 1 (y, 32 columns)
-      double fzn0 = 0.0, fzn1 = 0.0, fzn2 = 0.0;
+      fzl2 = F_zz<S>(B);
+    }
+    __syncthreads();  // plane kb-2 is read before its slot is loaded again
+  }
+  for (int k = kb; k <= ke; ++k) {
+    // planes k+3 (velocity) and k+2 (cell) into slots last read by an earlier step
+    if (k < ke) load_planes(k + 3, k + 2);
+    at_plane(k);
+    double ppx = 0.0, ppy = 0.0, ppz = 0.0;
+    if (OUT && in) {
+      if (k >= 1) {
+        ppx = __ldg(a.ppx + box_x(a, i, j, k));
+        if (j <= a.ny - 1) ppy = __ldg(a.ppy + box_y(a, i, j, k));
+      }
+      ppz = __ldg(a.ppz + box_z(a, i, j, k));
+    }
+    invert(k + 1);
+    // the cell's upper z faces stay in registers: the next plane's lower ones
+    double fzn0 = 0.0, fzn1 = 0.0, fzn2 = 0.0;
+    if constexpr (S != 5) {
       if (in) {
         const Met g(a, i, j, k);
-        fx[(0 * kTY + ty) * (kTX + 1) + tx + 1] = F_xx<S>(A);
-        fx[(1 * kTY + ty) * (kTX + 1) + tx + 1] = F_yx<S>(A, g);
-        fx[(2 * kTY + ty) * (kTX + 1) + tx + 1] = F_zx<S>(A);
-        fy[(0 * (kTY + 1) + ty + 1) * kTX + tx] = F_xy<S>(A);
-        fy[(1 * (kTY + 1) + ty + 1) * kTX + tx] = F_yy<S>(A);
-        fy[(2 * (kTY + 1) + ty + 1) * kTX + tx] = F_zy<S>(A);
         fzn0 = F_xz<S>(A);
         fzn1 = F_yz<S>(A, g);
         fzn2 = F_zz<S>(A);
-        if (k == kb) {  // the chunk's first lower z faces (ux, uy need none at k = 0)
-          const SAcc B = A.down();
-          if (kb > 0) {
-            fzl0 = F_xz<S>(B);
-            fzl1 = F_yz<S>(B, g);
-          }
-          fzl2 = F_zz<S>(B);
-        }
       }
-      if (ty == 0 && tx < kTY && j0 + tx <= a.ny) {
-        const SAcc E = A.shifted(-1 - tx, tx);
-        const Met ge(a, i0 - 1, j0 + tx, k);
-        fx[(0 * kTY + tx) * (kTX + 1)] = F_xx<S>(E);
-        fx[(1 * kTY + tx) * (kTX + 1)] = F_yx<S>(E, ge);
-        fx[(2 * kTY + tx) * (kTX + 1)] = F_zx<S>(E);
-      } else if (ty == 1 && i0 + tx <= a.nx) {
-        const SAcc E = A.shifted(0, -2);
-        fy[(0 * (kTY + 1)) * kTX + tx] = F_xy<S>(E);
-        fy[(1 * (kTY + 1)) * kTX + tx] = F_yy<S>(E);
-        fy[(2 * (kTY + 1)) * kTX + tx] = F_zy<S>(E);
-      }
-      __syncthreads();
-      if (in) {
-        const Met g(a, i, j, k);
-        const double irc = 1.0 / A.r(0, 0, 0);
-        auto cxd = [&](int c) { return fx[(c * kTY + ty) * (kTX + 1) + tx + 1] - fx[(c * kTY + ty) * (kTX + 1) + tx]; };
-        auto cyd = [&](int c) { return fy[(c * (kTY + 1) + ty + 1) * kTX + tx] - fy[(c * (kTY + 1) + ty) * kTX + tx]; };
-        if (k >= 1) {
-          const double ivx = 0.5 * (1.0 / A.r(1, 0, 0) + irc);
-          emit_x<OUT>(a, i, j, k, tail_x(A, g, ivx, cxd(0), cyd(0), fzn0 - fzl0), A.u(0, 0, 0), ivx);
-          if (j <= a.ny - 1)
-            emit_y<OUT>(a, i, j, k, tail_y(A, g, 0.5 * (1.0 / A.r(0, 1, 0) + irc), cxd(1), cyd(1), fzn1 - fzl1),
-                        A.v(0, 0, 0));
-        }
-        emit_z<OUT>(a, i, j, k, tail_z(A, g, 0.5 * (1.0 / A.r(0, 0, 1) + irc), cxd(2), cyd(2), fzn2 - fzl2),
-                    A.w(0, 0, 0));
-      }
-      fzl0 = fzn0;
-      fzl1 = fzn1;
-      fzl2 = fzn2;
     }
+    if (in) {
+      const double irc = A.r(0, 0, 0);  // 1/rho of the own cell, shared by the three components
+      const Met g(a, i, j, k);
+      if (k >= 1) {
+        const double ivx = 0.5 * (A.r(1, 0, 0) + irc);
+        emit_x<OUT>(a, i, j, k, phi_x<S, S == 5>(A, g, ivx, fzn0 - fzl0), A.u(0, 0, 0), ivx, ppx);
+        if (j <= a.ny - 1)
+          emit_y<OUT>(a, i, j, k, phi_y<S, S == 5>(A, g, 0.5 * (A.r(0, 1, 0) + irc), fzn1 - fzl1), A.v(0, 0, 0),
+                      ppy);
+      }
+      emit_z<OUT>(a, i, j, k, phi_z<S, S == 5>(A, g, 0.5 * (A.r(0, 0, 1) + irc), fzn2 - fzl2), A.w(0, 0, 0), ppz);
+    }
+    fzl0 = fzn0;
+    fzl1 = fzn1;
+    fzl2 = fzn2;
     cp_async_wait_all();
     __syncthreads();
   }
 }
 
 __host__ __device__ constexpr size_t tiled_smem_bytes(int S) {
-  return sizeof(double) * (3 * kRV * kNV + 2 * kRC * kNC + (S == 5 ? kRC * kNC : 0) +
-                           (share_faces(S) ? 3 * kTY * (kTX + 1) + 3 * (kTY + 1) * kTX : 0));
+  return sizeof(double) * (3 * ring_v(S) * kNV + 2 * kRC * kNC + (S == 5 ? kRC * kNC : 0));
 }
 
 // the x component's face i = 0 (the periodic duplicate of i = nx, computed
@@ -624,7 +585,8 @@ __global__ void __launch_bounds__(kMT) k_momentum_fluxes_i0(MomArgs a) {
   if (j > a.ny) return;
   const GAcc A(a, 0, j, k);
   const double ivx = 0.5 * (1.0 / A.r(1, 0, 0) + 1.0 / A.r(0, 0, 0));
-  emit_x<OUT>(a, 0, j, k, phi_x<S>(A, Met(a, 0, j, k), ivx), A.u(0, 0, 0), ivx);
+  const double pp = OUT ? __ldg(a.ppx + box_x(a, 0, j, k)) : 0.0;
+  emit_x<OUT>(a, 0, j, k, phi_x<S, true>(A, Met(a, 0, j, k), ivx, 0.0), A.u(0, 0, 0), ivx, pp);
 }
 
 // The out-of-place form leaves the elements outside the equation boxes to
@@ -677,7 +639,7 @@ __global__ void __launch_bounds__(256) k_copy_outside_box(CmpArgs a) {
 }
 
 template <int S, bool OUT>
-void launch_fluxes(const MomArgs &a, cudaStream_t st) {
+void launch_fluxes(MomArgs a, cudaStream_t st) {
   static bool attr[64] = {};  // per device: the attribute belongs to the device's context
   int dev = 0;
   cudaGetDevice(&dev);
@@ -686,7 +648,11 @@ void launch_fluxes(const MomArgs &a, cudaStream_t st) {
                          (int)tiled_smem_bytes(S));
     if (dev < 64) attr[dev] = true;
   }
-  const dim3 blk(kTX, kTY), grid((a.nx + kTX - 1) / kTX, (a.ny + kTY - 1) / kTY, (a.nz + 1 + kKC - 1) / kKC);
+  const dim3 blk(kTX, kTY), tiles((a.nx + kTX - 1) / kTX, (a.ny + kTY - 1) / kTY);
+  // a fixed 64 planes per block left 39 blocks for the chip on 96x100x48 (0.155
+  // ms; now 0.078) and a fifth chunk of one plane on 512x384x256 (2.35 ms; now 2.32)
+  a.kc = march_chunk((long)tiles.x * tiles.y, a.nz + 1, 148L * kMomBlocks, 5);
+  const dim3 grid(tiles.x, tiles.y, (a.nz + a.kc) / a.kc);
   k_momentum_fluxes<S, OUT><<<grid, blk, tiled_smem_bytes(S), st>>>(a);
   k_momentum_fluxes_i0<S, OUT><<<dim3((a.ny + kMT - 1) / kMT, a.nz), kMT, 0, st>>>(a);
 }
@@ -713,7 +679,7 @@ struct MomUpd {
 };
 
 __device__ __forceinline__ void update_x(const MomUpd &a, const MomArgs &b, int i, int j, int k) {
-  const long o = at(a.Lux, i, j, k), q = box_x(b, i, j, k);
+  const int o = at32(a.Lux, i, j, k), q = box_x(b, i, j, k);
   double u = a.ux[o] + a.dt * (a.gamma * a.phx[q] + a.xi * a.ppx[q]);
   const double invrho = 0.5 * (1.0 / a.rho[at(a.Lc, i + 1, j, k)] + 1.0 / a.rho[at(a.Lc, i, j, k)]);
   const double st = a.stx ? a.stx[at(a.Lsx, i, j, k)] : 0.0;
@@ -732,13 +698,13 @@ __global__ void __launch_bounds__(kMT) k_momentum_update(MomUpd a) {
     update_x(a, b, i, j, k);
     if (i == a.nx) update_x(a, b, 0, j, k);
     if (j <= a.ny - 1) {
-      const long o = at(a.Luy, i, j, k), q = box_y(b, i, j, k);
+      const int o = at32(a.Luy, i, j, k), q = box_y(b, i, j, k);
       double u = a.uy[o] + a.dt * (a.gamma * a.phy[q] + a.xi * a.ppy[q]);
       const double st = a.sty ? a.sty[at(a.Lsy, i, j, k)] : 0.0;
       a.uy[o] = u + a.invrho0 * a.r * st + a.r * a.g;
     }
   }
-  const long o = at(a.Luz, i, j, k), q = box_z(b, i, j, k);
+  const int o = at32(a.Luz, i, j, k), q = box_z(b, i, j, k);
   double u = a.uz[o] + a.dt * (a.gamma * a.phz[q] + a.xi * a.ppz[q]);
   const double st = a.stz ? a.stz[at(a.Lsz, i, j, k)] : 0.0;
   a.uz[o] = u + a.invrho0 * a.r * st;
