@@ -3,7 +3,7 @@
 // computeFlowRate (the ux flux), and setFlowRate's uniform shift of ux.
 // A sum runs over the ux faces i = 0..nx-1, j = 1..ny, k = 1..nz with the
 // staggered volume Vsx(i,j,k) = dxc(i+1)*dyf(j)*dzf(k) (grid.f90:812-838):
-// one block per (j, k) row into a partial, then one block adds the partials
+// one warp per (j, k) row into a partial, then one block adds the partials
 // in a fixed order, so a sum is the same on every call (its order differs
 // from the reference's sequential loop: agreement to rounding).
 #include <cuda_runtime.h>
@@ -16,28 +16,31 @@ namespace {
 
 constexpr int kRT = 128;
 
+constexpr int kRW = 8;  // rows per block, one per warp
+
+// A warp adds one row, four loads in flight per lane, and folds it by shuffles
+// (0.114 ms on 512x384x256 with a block of 128 threads and a shared-memory tree
+// per row; now 0.084, 0.061 at the copy bandwidth).
 template <int MODE>  // 0: 0.5*(rho(i+1)+rho(i)), 1: ux(i)
-__global__ void __launch_bounds__(kRT) k_face_sum_rows(const double *__restrict__ f, Lay L,
-                                                       const double *__restrict__ dxc, const double *__restrict__ dyf,
-                                                       const double *__restrict__ dzf, int nx, int ny,
-                                                       double *__restrict__ part) {
-  const int j = blockIdx.x + 1, k = blockIdx.y + 1;
+__global__ void __launch_bounds__(32 * kRW) k_face_sum_rows(const double *__restrict__ f, Lay L,
+                                                            const double *__restrict__ dxc,
+                                                            const double *__restrict__ dyf,
+                                                            const double *__restrict__ dzf, int nx, int ny, int nz,
+                                                            double *__restrict__ part) {
+  const int lane = threadIdx.x & 31;
+  const long row = (long)blockIdx.x * kRW + (threadIdx.x >> 5);
+  if (row >= (long)ny * nz) return;
+  const int j = (int)(row % ny) + 1, k = (int)(row / ny) + 1;
   const double dy = dyf[j - 1], dz = dzf[k - 1];
+  const double *r = f + at(L, 0, j, k);
   double s = 0.0;
-  for (int i = threadIdx.x; i < nx; i += kRT) {
-    const long o = at(L, i, j, k);
-    const double x = MODE == 0 ? 0.5 * (f[o + 1] + f[o]) : f[o];
-    const double dV = dxc[i] * dy * dz;  // dxc(i+1)*dyf(j)*dzf(k)
-    s += x * dV;
+#pragma unroll 4
+  for (int i = lane; i < nx; i += 32) {
+    const double x = MODE == 0 ? 0.5 * (r[i + 1] + r[i]) : r[i];
+    s += x * (dxc[i] * dy * dz);  // dxc(i+1)*dyf(j)*dzf(k)
   }
-  __shared__ double red[kRT];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = kRT / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[(long)(k - 1) * ny + (j - 1)] = red[0];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) part[row] = s;
 }
 
 __global__ void __launch_bounds__(1024) k_sum_partials(const double *__restrict__ part, long n,
@@ -66,9 +69,9 @@ __global__ void __launch_bounds__(kRT) k_add_ux(double *__restrict__ ux, Lay L, 
 
 void launch_face_sum(int mode, const double *f, Lay L, const double *dxc, const double *dyf, const double *dzf, int nx,
                      int ny, int nz, double *part, double *out, cudaStream_t st) {
-  const dim3 grid(ny, nz);
-  if (mode == 0) k_face_sum_rows<0><<<grid, kRT, 0, st>>>(f, L, dxc, dyf, dzf, nx, ny, part);
-  else k_face_sum_rows<1><<<grid, kRT, 0, st>>>(f, L, dxc, dyf, dzf, nx, ny, part);
+  const unsigned grid = (unsigned)(((long)ny * nz + kRW - 1) / kRW);
+  if (mode == 0) k_face_sum_rows<0><<<grid, 32 * kRW, 0, st>>>(f, L, dxc, dyf, dzf, nx, ny, nz, part);
+  else k_face_sum_rows<1><<<grid, 32 * kRW, 0, st>>>(f, L, dxc, dyf, dzf, nx, ny, nz, part);
   k_sum_partials<<<1, 1024, 0, st>>>(part, (long)ny * nz, out);
 }
 
