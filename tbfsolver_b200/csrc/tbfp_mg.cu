@@ -108,6 +108,15 @@ __device__ __forceinline__ void block_sum2(double a, double b, double *out_a, do
 // red and black sweeps of a smoothing call give sum(p) for correctFullNeumann
 // without another pass).  A wall cell's clamped y neighbour is the cell
 // itself, so a sweep also reads cells of its own colour there.
+// A block's walk takes kRbU rows at a time with all their loads in front: a sweep
+// reads no cell that it writes (but a wall cell itself), which the compiler cannot
+// know, so row by row each row's loads wait for the stores of the one before.
+// 256x256x128, finest level: 0.030 ms a sweep with two rows (0.039 with one and
+// 64-bit indices, 0.034 with one, 0.032 with four: 80 registers).  A walk of one row
+// takes the one-row form.  A fused red + black pass (64 x 14 tiles marching up z,
+// planes in shared memory) read the level half as often and took as long, 0.078 ms:
+// 16 warps per SM, a barrier per plane and a quarter of halo cells.
+template <int kRbU>
 __global__ void __launch_bounds__(kWalkX) k_rbgs_colour(MgLev L, float *__restrict__ p,
                                                        const float *__restrict__ q,
                                                        const float *__restrict__ beta, int colour,
@@ -116,21 +125,48 @@ __global__ void __launch_bounds__(kWalkX) k_rbgs_colour(MgLev L, float *__restri
   const int nx = L.nx, ny = L.ny, nz = L.nz, k = w.k;
   double acc = 0.0;
   if (w.i < (nx + 1) / 2) {
-    for (int j = w.j0; j < w.j1; ++j) {
-      // colour of 1-based (i+1, j+1, k+1) is (i + j + k + 3) mod 2, so the row's
-      // first 0-based index of this colour is (colour + j + k + 1) mod 2
-      const int ii = 2 * w.i + ((colour + j + k + 1) & 1);
-      if (ii >= nx) continue;
-      auto at3 = [&](int a, int b, int c) { return (c * ny + b) * nx + a; };
-      const Coef<float> c = coef<float>(L, beta, ii, j, k);
-      const float den = c.aR + c.aL + c.aT + c.aB + c.aF + c.aK;
-      const float pR = p[at3(wrap(ii + 1, nx), j, k)], pL = p[at3(wrap(ii - 1, nx), j, k)];
-      const float pT = p[at3(ii, clampi(j + 1, ny), k)], pB = p[at3(ii, clampi(j - 1, ny), k)];
-      const float pF = p[at3(ii, j, wrap(k + 1, nz))], pK = p[at3(ii, j, wrap(k - 1, nz))];
-      const float v =
-          (-q[at3(ii, j, k)] + (c.aR * pR + c.aL * pL) + (c.aT * pT + c.aB * pB) + (c.aF * pF + c.aK * pK)) / den;
-      p[at3(ii, j, k)] = v;
-      acc += v;
+    const int kf = wrap(k + 1, nz) * ny * nx, kk = wrap(k - 1, nz) * ny * nx, k0 = k * ny * nx;
+    const float zf = 0.5f * L.invz1[k], zk = 0.5f * L.invz2[k];  // halving a metric is exact
+    for (int j0 = w.j0; j0 < w.j1; j0 += kRbU) {
+      float b[kRbU][7], v[kRbU][6], qv[kRbU];
+#pragma unroll
+      for (int u = 0; u < kRbU; ++u) {
+        // colour of 1-based (i+1, j+1, k+1) is (i + j + k + 3) mod 2, so the row's
+        // first 0-based index of this colour is (colour + j + k + 1) mod 2
+        const int j = min(j0 + u, w.j1 - 1), i = 2 * w.i + ((colour + j + k + 1) & 1);
+        const int ii = min(i, nx - 1);
+        const int o = k0 + j * nx, xr = o + wrap(ii + 1, nx), xl = o + wrap(ii - 1, nx);
+        const int yt = k0 + clampi(j + 1, ny) * nx + ii, yb = k0 + clampi(j - 1, ny) * nx + ii;
+        const int f = kf + j * nx + ii, g = kk + j * nx + ii;
+        b[u][0] = beta[o + ii];
+        b[u][1] = beta[xr];
+        b[u][2] = beta[xl];
+        b[u][3] = beta[yt];
+        b[u][4] = beta[yb];
+        b[u][5] = beta[f];
+        b[u][6] = beta[g];
+        v[u][0] = p[xr];
+        v[u][1] = p[xl];
+        v[u][2] = p[yt];
+        v[u][3] = p[yb];
+        v[u][4] = p[f];
+        v[u][5] = p[g];
+        qv[u] = q[o + ii];
+      }
+#pragma unroll
+      for (int u = 0; u < kRbU; ++u) {
+        const int j = j0 + u, i = 2 * w.i + ((colour + j + k + 1) & 1);
+        if (j >= w.j1 || i >= nx) continue;
+        const float c = b[u][0];
+        const float aR = (b[u][1] + c) * (0.5f * L.invx1[i]), aL = (c + b[u][2]) * (0.5f * L.invx2[i]);
+        const float aT = (b[u][3] + c) * (0.5f * L.invy1[j]), aB = (c + b[u][4]) * (0.5f * L.invy2[j]);
+        const float aF = (b[u][5] + c) * zf, aK = (c + b[u][6]) * zk;
+        const float den = aR + aL + aT + aB + aF + aK;
+        const float x =
+            (-qv[u] + (aR * v[u][0] + aL * v[u][1]) + (aT * v[u][2] + aB * v[u][3]) + (aF * v[u][4] + aK * v[u][5])) / den;
+        p[k0 + j * nx + i] = x;
+        acc += x;
+      }
     }
   }
   if (sum) block_sum2(acc, 0.0, sum, nullptr);  // sum is uniform over the grid
@@ -143,17 +179,83 @@ __global__ void __launch_bounds__(kMgThreads) k_sub_mean(float *__restrict__ p, 
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) p[t] -= avg;
 }
 
-// res = q - L p (computeResiduals, rbgs.f90:308-317); optional sum res^2, sum q^2
+// res = q - L p (computeResiduals, rbgs.f90:308-317) of the 2 x 2 x 2 cells under
+// one coarse cell, one thread each, with p and beta read in pairs (x is even
+// everywhere below a coarser level): 44 loads for eight cells, and the residual
+// itself never goes to memory.  RESTRICT: their weighted sum into the coarse
+// level's q (restrictionOp3D); else their squares and those of q into nrm[0], nrm[1].
+// 256x256x128: 0.039 ms (norms 0.040), where a residual written cell by cell and
+// read back by the restriction took 0.070 + 0.007 ms, and the norm pass 0.070.
+constexpr int kResJ = 4;  // coarse rows per block of the norm form
+template <bool RESTRICT>
+__global__ void __launch_bounds__(kWalkX) k_residual8(MgLev F, const float *__restrict__ p, const float *__restrict__ q,
+                                                      const float *__restrict__ beta, MgLev C,
+                                                      float *__restrict__ coarse, double *__restrict__ nrm) {
+  const Walk w = walk(F.ny / 2);
+  const int nx = F.nx, ny = F.ny, nz = F.nz, I = w.i, K = w.k, x = 2 * I;
+  double rr = 0.0, qq = 0.0;
+  if (x < nx) {
+    const int xl = x > 0 ? x - 1 : nx - 1, xr = x + 2 < nx ? x + 2 : 0;
+    const int kk[4] = {wrap(2 * K - 1, nz), 2 * K, 2 * K + 1, wrap(2 * K + 2, nz)};
+    const float h = 0.5f;
+    const float ax0 = F.invx2[x], ax1 = F.invx1[x], ax2 = F.invx2[x + 1], ax3 = F.invx1[x + 1];
+    for (int J = w.j0; J < w.j1; ++J) {
+      const int jj[4] = {clampi(2 * J - 1, ny), 2 * J, 2 * J + 1, clampi(2 * J + 2, ny)};
+      auto row = [&](int b, int c) { return (kk[c] * ny + jj[b]) * nx; };
+      auto pair = [&](const float *a, int b, int c) { return *reinterpret_cast<const float2 *>(a + row(b, c) + x); };
+      float2 B[4][4], P[4][4];  // rows 2J-1..2J+2 of planes 2K-1..2K+2, the corners not read
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if ((b == 1 || b == 2) || (c == 1 || c == 2)) {
+            B[c][b] = pair(beta, b, c);
+            P[c][b] = pair(p, b, c);
+          }
+      float s = 0.0f;
+#pragma unroll
+      for (int c = 1; c < 3; ++c)
+#pragma unroll
+        for (int b = 1; b < 3; ++b) {
+          const int r = row(b, c);
+          const float bl = beta[r + xl], br = beta[r + xr], pl = p[r + xl], pr = p[r + xr];
+          const float2 qv = pair(q, b, c), bc = B[c][b], pc = P[c][b];
+          const float y1 = F.invy1[jj[b]], y2 = F.invy2[jj[b]], z1 = F.invz1[kk[c]], z2 = F.invz2[kk[c]];
+          auto cell = [&](float bcc, float pcc, float bL, float pL, float wl, float bR, float pR, float wr, float bT,
+                          float pT, float bB, float pB, float bF, float pF, float bK, float pK, float qc) {
+            const float aR = h * (bR + bcc) * wr, aL = h * (bcc + bL) * wl, aT = h * (bT + bcc) * y1,
+                        aB = h * (bcc + bB) * y2, aF = h * (bF + bcc) * z1, aK = h * (bcc + bK) * z2;
+            const float Lp = aR * (pR - pcc) - aL * (pcc - pL) + aT * (pT - pcc) - aB * (pcc - pB) + aF * (pF - pcc) -
+                             aK * (pcc - pK);
+            return qc - Lp;
+          };
+          const float r0 = cell(bc.x, pc.x, bl, pl, ax0, bc.y, pc.y, ax1, B[c][b + 1].x, P[c][b + 1].x, B[c][b - 1].x,
+                                P[c][b - 1].x, B[c + 1][b].x, P[c + 1][b].x, B[c - 1][b].x, P[c - 1][b].x, qv.x);
+          const float r1 = cell(bc.y, pc.y, bc.x, pc.x, ax2, br, pr, ax3, B[c][b + 1].y, P[c][b + 1].y, B[c][b - 1].y,
+                                P[c][b - 1].y, B[c + 1][b].y, P[c + 1][b].y, B[c - 1][b].y, P[c - 1][b].y, qv.y);
+          if constexpr (RESTRICT) {
+            const float yz = C.ry[2 * J + b - 1] * C.rz[2 * K + c - 1];
+            s += (C.rx[2 * I] * yz) * r0 + (C.rx[2 * I + 1] * yz) * r1;
+          } else {
+            rr += (double)r0 * r0 + (double)r1 * r1;
+            qq += (double)qv.x * qv.x + (double)qv.y * qv.y;
+          }
+        }
+      if constexpr (RESTRICT) coarse[(K * (ny / 2) + J) * (nx / 2) + I] = s;
+    }
+  }
+  if constexpr (!RESTRICT) block_sum2(rr, qq, nrm, nrm + 1);
+}
+
+// Norms of a finest level that has no coarser one (a single level).
 __global__ void __launch_bounds__(kMgThreads) k_mg_residual(MgLev L, const float *__restrict__ p,
                                                            const float *__restrict__ q,
-                                                           const float *__restrict__ beta, float *__restrict__ res,
-                                                           double *__restrict__ nrm) {
+                                                           const float *__restrict__ beta, double *__restrict__ nrm) {
   const Walk w = walk(L.ny);
   const int nx = L.nx, ny = L.ny, nz = L.nz, i = w.i, k = w.k;
   double rr = 0.0, qq = 0.0;
   if (i < nx) {
     auto at3 = [&](int a, int b, int c) { return (c * ny + b) * nx + a; };
-#pragma unroll 4
     for (int j = w.j0; j < w.j1; ++j) {
       const int t = at3(i, j, k);
       const Coef<float> c = coef<float>(L, beta, i, j, k);
@@ -162,12 +264,11 @@ __global__ void __launch_bounds__(kMgThreads) k_mg_residual(MgLev L, const float
                        c.aT * (p[at3(i, clampi(j + 1, ny), k)] - pc) - c.aB * (pc - p[at3(i, clampi(j - 1, ny), k)]) +
                        c.aF * (p[at3(i, j, wrap(k + 1, nz))] - pc) - c.aK * (pc - p[at3(i, j, wrap(k - 1, nz))]);
       const float v = q[t] - Lp;
-      res[t] = v;
       rr += (double)v * v;
       qq += (double)q[t] * q[t];
     }
   }
-  if (nrm) block_sum2(rr, qq, nrm, nrm + 1);
+  block_sum2(rr, qq, nrm, nrm + 1);
 }
 
 // restrictionOp3D (interpolation.f90:80-124): coarse = sum of the 8 children with
@@ -390,6 +491,160 @@ __global__ void k_coarse_apply(MgLev L, const double *__restrict__ M, int n1, co
 }
 
 // ---------------------------------------------------------------------------
+// The coarse end of a V-cycle, levels l0 .. last, in one launch of one CTA with
+// every level's p, q and beta in shared memory: zero-start smoothing, residual and
+// restriction down to the coarsest level, its bordered inverse applied, then
+// prolongation and smoothing back up.  A launch per step cost 2 to 3 us each, 13 of
+// them for the 16x16x8 and 8x8x4 levels of 256x256x128; the CTA takes 0.039 ms for
+// both.  With the 32x32x16 level in it as well (220 KB) it took 0.188 ms: a sweep of
+// 16,384 cells is too much for one SM.
+// q of level l0 comes from the restriction before, p of level l0 and the pending
+// sum of its last smoothing go back to memory.
+// ---------------------------------------------------------------------------
+constexpr int kMgMaxLevels = 16, kTailThreads = 1024;
+constexpr size_t kTailSmem = 64 * 1024;
+constexpr int kTailCoarse = 512;  // unknowns of the coarsest system whose inverse one SM applies (2 MB of it)
+struct MgTail {
+  int n;  // levels, the last one the coarsest
+  int n_pre, n_post;
+  MgLev L[kMgMaxLevels];
+  const float *beta[kMgMaxLevels];
+  const float *q0;  // q of the first level
+  float *p0;        // its p
+  double *post0;    // its pending sum
+  const double *M;  // inverse of the coarsest system
+  int n1;
+};
+
+__device__ double tail_sum(double v) {  // the same sum in every thread
+  __shared__ double red[kTailThreads / 32];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();  // the sum before has been read
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+  for (int w = 0; w < kTailThreads / 32; ++w) s += red[w];
+  return s;
+}
+
+__global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_constant__ MgTail T) {
+  extern __shared__ __align__(16) float ts[];
+  const int tid = threadIdx.x, last = T.n - 1;
+  float *p[kMgMaxLevels], *q[kMgMaxLevels], *bt[kMgMaxLevels];
+  {
+    float *f = ts;
+    for (int l = 0; l < T.n; ++l) {
+      const int n = T.L[l].nx * T.L[l].ny * T.L[l].nz;
+      p[l] = f;
+      q[l] = f + n;
+      bt[l] = f + 2 * n;  // not kept for the coarsest level
+      f += l < last ? 3 * n : 2 * n;
+      if (l < last)
+        for (int t = tid; t < n; t += kTailThreads) bt[l][t] = T.beta[l][t];
+      if (l == 0)
+        for (int t = tid; t < n; t += kTailThreads) q[l][t] = T.q0[t];
+    }
+  }
+  // one smoothing call; returns the sum of p (its mean is removed by the caller)
+  auto smooth = [&](int l, int iters, bool reset) {
+    const MgLev &L = T.L[l];
+    const int nx = L.nx, ny = L.ny, nz = L.nz, n = nx * ny * nz, hx = nx / 2;
+    if (reset)
+      for (int t = tid; t < n; t += kTailThreads) p[l][t] = 0.0f;
+    __syncthreads();
+    const float *B = bt[l], *Q = q[l];
+    float *P = p[l];
+    for (int it = 0; it < 2 * iters; ++it) {
+      for (int t = tid; t < n / 2; t += kTailThreads) {
+        const int r = t / hx, k = r / ny, j = r - k * ny, i = 2 * (t - r * hx) + (((it & 1) + j + k + 1) & 1);
+        const Coef<float> c = coef<float>(L, B, i, j, k);
+        const int o = r * nx, sk = nx * ny;
+        const float den = c.aR + c.aL + c.aT + c.aB + c.aF + c.aK;
+        const float pR = P[o + wrap(i + 1, nx)], pL = P[o + wrap(i - 1, nx)];
+        const float pT = P[(k * ny + clampi(j + 1, ny)) * nx + i], pB = P[(k * ny + clampi(j - 1, ny)) * nx + i];
+        const float pF = P[wrap(k + 1, nz) * sk + j * nx + i], pK = P[wrap(k - 1, nz) * sk + j * nx + i];
+        P[o + i] = (-Q[o + i] + (c.aR * pR + c.aL * pL) + (c.aT * pT + c.aB * pB) + (c.aF * pF + c.aK * pK)) / den;
+      }
+      __syncthreads();
+    }
+    if (iters == 0) return 0.0;
+    double s = 0.0;
+    for (int t = tid; t < n; t += kTailThreads) s += P[t];
+    return tail_sum(s);
+  };
+  double pre[kMgMaxLevels];
+  for (int l = 0; l < last; ++l) {
+    pre[l] = smooth(l, T.n_pre, true);
+    // residual of the eight cells under each coarse cell, restricted
+    const MgLev &F = T.L[l], &C = T.L[l + 1];
+    const int nc = C.nx * C.ny * C.nz;
+    for (int t = tid; t < nc; t += kTailThreads) {
+      const int r = t / C.nx, K = r / C.ny, J = r - K * C.ny, I = t - r * C.nx;
+      float s = 0.0f;
+      for (int e = 0; e < 8; ++e) {
+        const int i = 2 * I + (e & 1), j = 2 * J + (e >> 1 & 1), k = 2 * K + (e >> 2);
+        const Coef<float> c = coef<float>(F, bt[l], i, j, k);
+        auto P = [&](int a, int b, int d) { return p[l][(d * F.ny + b) * F.nx + a]; };
+        const float pc = P(i, j, k);
+        const float Lp = c.aR * (P(wrap(i + 1, F.nx), j, k) - pc) - c.aL * (pc - P(wrap(i - 1, F.nx), j, k)) +
+                         c.aT * (P(i, clampi(j + 1, F.ny), k) - pc) - c.aB * (pc - P(i, clampi(j - 1, F.ny), k)) +
+                         c.aF * (P(i, j, wrap(k + 1, F.nz)) - pc) - c.aK * (pc - P(i, j, wrap(k - 1, F.nz)));
+        s += (C.rx[i] * C.ry[j]) * C.rz[k] * (q[l][(k * F.ny + j) * F.nx + i] - Lp);
+      }
+      q[l + 1][t] = s;
+    }
+    __syncthreads();
+  }
+  {  // p = K^-1 (-V q) on the coarsest level (k_coarse_apply)
+    const MgLev &L = T.L[last];
+    const int n = T.n1 - 1, ld = 2 * T.n1, lane = tid & 31;
+    for (int t = tid; t < n; t += kTailThreads) {
+      const int r = t / L.nx, k = r / L.ny;
+      q[last][t] *= -(L.vx[t - r * L.nx] * L.vy[r - k * L.ny] * L.vz[k]);
+    }
+    __syncthreads();
+    for (int r = tid >> 5; r < n; r += kTailThreads / 32) {
+      const double *row = T.M + (long)coarse_perm(r, n) * ld + T.n1;
+      double acc = 0.0;
+#pragma unroll 4
+      for (int c = lane; c < n; c += 32) acc += row[coarse_perm(c, n)] * (double)q[last][c];
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) p[last][r] = (float)acc;
+    }
+    __syncthreads();
+  }
+  double post = 0.0;  // pending sum of the level below
+  for (int l = last - 1; l >= 0; --l) {
+    const MgLev &F = T.L[l], &C = T.L[l + 1];
+    const int n = F.nx * F.ny * F.nz;
+    const float mf = (float)(pre[l] / (double)n), mc = (float)(post / (double)(C.nx * C.ny * C.nz));
+    for (int t = tid; t < n; t += kTailThreads) {
+      const int r = t / F.nx, k = r / F.ny, j = r - k * F.ny, i = t - r * F.nx;
+      const int ih = (i + 1) / 2 - 1, jh = (j + 1) / 2 - 1, kh = (k + 1) / 2 - 1;
+      const int xa = wrap(ih, C.nx), xb = wrap(ih + 1, C.nx), ya = clampi(jh, C.ny), yb = clampi(jh + 1, C.ny);
+      const int za = wrap(kh, C.nz), zb = wrap(kh + 1, C.nz);
+      const float x0 = F.px[2 * i], x1 = F.px[2 * i + 1], y0 = F.py[2 * j], y1 = F.py[2 * j + 1];
+      const float z0 = F.pz[2 * k], z1 = F.pz[2 * k + 1];
+      auto c = [&](int a, int b, int d) { return p[l + 1][(d * C.ny + b) * C.nx + a]; };
+      float s = (x0 * y0) * z0 * c(xa, ya, za);
+      s += (x1 * y0) * z0 * c(xb, ya, za);
+      s += (x0 * y1) * z0 * c(xa, yb, za);
+      s += (x1 * y1) * z0 * c(xb, yb, za);
+      s += (x0 * y0) * z1 * c(xa, ya, zb);
+      s += (x1 * y0) * z1 * c(xb, ya, zb);
+      s += (x0 * y1) * z1 * c(xa, yb, zb);
+      s += (x1 * y1) * z1 * c(xb, yb, zb);
+      p[l][t] = (p[l][t] - mf) + (s - mc);
+    }
+    __syncthreads();
+    post = smooth(l, T.n_post, false);
+  }
+  const int n0 = T.L[0].nx * T.L[0].ny * T.L[0].nz;
+  for (int t = tid; t < n0; t += kTailThreads) T.p0[t] = p[0][t];
+  if (tid == 0 && T.post0) *T.post0 = post;
+}
+
+// ---------------------------------------------------------------------------
 // FP64 PCG kernels on the finest level.  psi uses the caller's layout (halo
 // hd_psi), q and beta theirs; r, d, qv are dense.
 // ---------------------------------------------------------------------------
@@ -401,15 +656,17 @@ struct Fine {
 };
 
 __device__ __forceinline__ Coef<double> coef64(const Fine &F, int i, int j, int k) {
-  auto b = [&](int a, int bb, int c) { return F.beta[at(F.Lb, a + 1, bb + 1, c + 1)]; };
-  const double bc = b(i, j, k);
+  // 32-bit offsets: every array holds fewer than 2^31 elements
+  const int sj = (int)F.Lb.sj, sk = (int)F.Lb.sk;
+  const double *b = F.beta + ((i + 1 - F.Lb.ilo) + (j + 1 - F.Lb.jlo) * sj + (k + 1 - F.Lb.klo) * sk);
+  const double bc = b[0];
   Coef<double> c;
-  c.aR = 0.5 * (b(wrap(i + 1, F.nx), j, k) + bc) * F.ix1[i];
-  c.aL = 0.5 * (bc + b(wrap(i - 1, F.nx), j, k)) * F.ix2[i];
-  c.aT = 0.5 * (b(i, clampi(j + 1, F.ny), k) + bc) * F.iy1[j];
-  c.aB = 0.5 * (bc + b(i, clampi(j - 1, F.ny), k)) * F.iy2[j];
-  c.aF = 0.5 * (b(i, j, wrap(k + 1, F.nz)) + bc) * F.iz1[k];
-  c.aK = 0.5 * (bc + b(i, j, wrap(k - 1, F.nz))) * F.iz2[k];
+  c.aR = 0.5 * (b[wrap(i + 1, F.nx) - i] + bc) * F.ix1[i];
+  c.aL = 0.5 * (bc + b[wrap(i - 1, F.nx) - i]) * F.ix2[i];
+  c.aT = 0.5 * (b[(clampi(j + 1, F.ny) - j) * sj] + bc) * F.iy1[j];
+  c.aB = 0.5 * (bc + b[(clampi(j - 1, F.ny) - j) * sj]) * F.iy2[j];
+  c.aF = 0.5 * (b[(wrap(k + 1, F.nz) - k) * sk] + bc) * F.iz1[k];
+  c.aK = 0.5 * (bc + b[(wrap(k - 1, F.nz) - k) * sk]) * F.iz2[k];
   return c;
 }
 
@@ -622,7 +879,7 @@ struct MgSolver::Impl {
   struct Level {
     int nx, ny, nz;
     long n;
-    float *p = nullptr, *q = nullptr, *beta = nullptr, *res = nullptr;
+    float *p = nullptr, *q = nullptr, *beta = nullptr;
     float *tab = nullptr;  // invx1, invx2, invy1, invy2, invz1, invz2, vx, vy, vz, rx, ry, rz, px, py, pz
     MgLev L{};
   };
@@ -641,7 +898,9 @@ struct MgSolver::Impl {
   int *fail = nullptr;
   std::vector<void *> allocs;
   size_t bytes = 0;
+  int tail = 0;                      // first level of k_mg_tail (the number of levels: none)
   cudaGraphExec_t vgraph = nullptr;  // one V-cycle from the finest level
+  cudaGraphExec_t zgraph = nullptr;  // the first V-cycle of a solve: p starts at 0
   bool graph_failed = false;
 
   template <typename T>
@@ -656,6 +915,7 @@ struct MgSolver::Impl {
   }
   ~Impl() {
     if (vgraph) cudaGraphExecDestroy(vgraph);
+    if (zgraph) cudaGraphExecDestroy(zgraph);
     for (void *p : allocs) cudaFree(p);
   }
 };
@@ -706,7 +966,6 @@ int MgSolver::init(const tbfp_mg_params &prm, int nx, int ny, int nz, const doub
     ck(m.alloc(&L.p, L.n));
     ck(m.alloc(&L.q, L.n));
     ck(m.alloc(&L.beta, L.n));
-    ck(m.alloc(&L.res, L.n));
     // tables
     std::vector<float> t;
     auto put = [&](const std::vector<double> &v) {
@@ -791,6 +1050,16 @@ int MgSolver::init(const tbfp_mg_params &prm, int nx, int ny, int nz, const doub
     G.py = L.tab + o[13];
     G.pz = L.tab + o[14];
   }
+  // the coarse levels small enough for one SM (k_mg_tail), if the coarsest system is
+  m.tail = prm.n_levels;
+  if (m.n1 <= kTailCoarse)
+    for (int l = prm.n_levels - 1; l >= 1; --l) {
+    size_t b = 8 * (size_t)m.lv.back().n;
+    for (int r = l; r + 1 < prm.n_levels; ++r) b += 12 * (size_t)m.lv[r].n;
+    if (b > kTailSmem || prm.n_levels - l > kMgMaxLevels) break;
+    m.tail = l;
+  }
+  ck(cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
   // FP64 fine tables from the caller's metrics (the reference's own values)
   std::vector<double> x1(nx), x2(nx), y1(ny), y2(ny), z1(nz), z2(nz);
   for (int i = 0; i < nx; ++i) {
@@ -843,39 +1112,64 @@ struct Run {
   // with adding a constant to p (the update is an average of neighbours, q
   // fixed), so removing the mean once after the last iteration gives the same
   // p.
-  // The mean of p is not removed in a separate pass: the last red and black
-  // sweeps of a smoothing call add sum(p) into `slot`, and the kernel that
-  // next combines p with another level (k_prolong_add) subtracts it; the
-  // residual in between does not need it (L p ignores constants).  Returns
-  // whether a sum is pending in `slot`.  With reset, p starts from 0.
+  // The mean of p is not removed in a separate pass: the last iteration of a
+  // smoothing call adds sum(p) into `slot`, and the kernel that next combines p
+  // with another level (k_prolong_add) subtracts it; the residual in between does
+  // not need it (L p ignores constants).  Returns whether a sum is pending in
+  // `slot`.  With reset, p starts from 0.
   bool rbgs(int l, int n_iter, bool reset, double *slot) {
     auto &L = m.lv[l];
     if (reset) k_fill<<<nblk_grid(L.n), kMgThreads, 0, st>>>(L.p, L.n, 0.0f);
     if (n_iter == 0) return false;
     for (int it = 0; it < n_iter; ++it) {
       const bool last = it == n_iter - 1;
-      const int J = last ? sum_rows((L.nx + 1) / 2, L.ny, L.nz) : rows_j((L.nx + 1) / 2, L.ny, L.nz, 4096, kMgJ);
       double *sum = last ? slot : nullptr;
-      k_rbgs_colour<<<wgrid((L.nx + 1) / 2, L.ny, L.nz, J), kWalkX, 0, st>>>(L.L, L.p, L.q, L.beta, 0, sum);
-      k_rbgs_colour<<<wgrid((L.nx + 1) / 2, L.ny, L.nz, J), kWalkX, 0, st>>>(L.L, L.p, L.q, L.beta, 1, sum);
+      const int J = last ? sum_rows((L.nx + 1) / 2, L.ny, L.nz) : rows_j((L.nx + 1) / 2, L.ny, L.nz, 4096, kMgJ);
+      for (int colour = 0; colour < 2; ++colour) {
+        const dim3 grid = wgrid((L.nx + 1) / 2, L.ny, L.nz, J);
+        if (J > 1) k_rbgs_colour<2><<<grid, kWalkX, 0, st>>>(L.L, L.p, L.q, L.beta, colour, sum);
+        else k_rbgs_colour<1><<<grid, kWalkX, 0, st>>>(L.L, L.p, L.q, L.beta, colour, sum);
+      }
     }
     return true;
   }
 
-  void vcycle(int l) {
+  void tail(int l0) {
+    const int last = (int)m.lv.size() - 1;
+    MgTail T{};
+    T.n = last - l0 + 1;
+    T.n_pre = m.prm.n_pre;
+    T.n_post = m.prm.n_post;
+    size_t bytes = 8 * (size_t)m.lv[last].n;
+    for (int l = l0; l <= last; ++l) {
+      T.L[l - l0] = m.lv[l].L;
+      T.beta[l - l0] = m.lv[l].beta;
+      if (l < last) bytes += 12 * (size_t)m.lv[l].n;
+    }
+    T.q0 = m.lv[l0].q;
+    T.p0 = m.lv[l0].p;
+    T.post0 = l0 < last && m.prm.n_post > 0 ? m.msum + 2 * l0 + 1 : nullptr;
+    T.M = m.Minv;
+    T.n1 = m.n1;
+    k_mg_tail<<<1, kTailThreads, bytes, st>>>(T);
+  }
+
+  // zero: p of the finest level starts at 0
+  void vcycle(int l, bool zero) {
     const int last = (int)m.lv.size() - 1;
     auto &L = m.lv[l];
     if (l == 0) cudaMemsetAsync(m.msum, 0, 2 * m.lv.size() * sizeof(double), st);
+    if (l == m.tail) return tail(l);
     if (l == last) {
       k_coarse_apply<<<(unsigned)((L.n * 32 + 255) / 256), 256, 0, st>>>(L.L, m.Minv, m.n1, L.q, L.p);
       return;  // the bordered solve gives sum(p) = 0: nothing pending
     }
     double *pre = m.msum + 2 * l, *post = m.msum + 2 * l + 1;
-    const bool hpre = rbgs(l, m.prm.n_pre, l != 0, pre);
-    k_mg_residual<<<wgrid(L.nx, L.ny, L.nz, rows_j(L.nx, L.ny, L.nz, 4096, 4)), kWalkX, 0, st>>>(L.L, L.p, L.q, L.beta, L.res, nullptr);
+    const bool hpre = rbgs(l, m.prm.n_pre, zero || l != 0, pre);
     auto &C = m.lv[l + 1];
-    k_restrict<<<wgrid(C.nx, C.ny, C.nz, rows_j(C.nx, C.ny, C.nz, 4096, 4)), kWalkX, 0, st>>>(L.L, C.L, L.res, C.q);
-    vcycle(l + 1);
+    k_residual8<true><<<wgrid(C.nx, C.ny, C.nz, rows_j(C.nx, C.ny, C.nz, 4096, 4)), kWalkX, 0, st>>>(
+        L.L, L.p, L.q, L.beta, C.L, C.q, nullptr);
+    vcycle(l + 1, false);
     const bool hcpost = l + 1 < last && m.prm.n_post > 0;
     k_prolong_add<<<wgrid(L.nx, L.ny, L.nz, rows_j(L.nx, L.ny, L.nz, 4096, 4)), kWalkX, 0, st>>>(
         L.L, C.L, C.p, L.p, hpre ? pre : nullptr, 1.0 / (double)L.n, hcpost ? m.msum + 2 * (l + 1) + 1 : nullptr,
@@ -889,7 +1183,10 @@ struct Run {
   int fine_residual(double *res, std::string *err) {
     auto &L = m.lv[0];
     cudaMemsetAsync(m.sc + 6, 0, 2 * sizeof(double), st);
-    k_mg_residual<<<wgrid(L.nx, L.ny, L.nz, kMgJ), kWalkX, 0, st>>>(L.L, L.p, L.q, L.beta, L.res, m.sc + 6);
+    if (m.lv.size() > 1)
+      k_residual8<false><<<wgrid(L.nx / 2, L.ny / 2, L.nz / 2, kResJ), kWalkX, 0, st>>>(L.L, L.p, L.q, L.beta, L.L,
+                                                                                       nullptr, m.sc + 6);
+    else k_mg_residual<<<wgrid(L.nx, L.ny, L.nz, kMgJ), kWalkX, 0, st>>>(L.L, L.p, L.q, L.beta, m.sc + 6);
     double v[2] = {0.0, 0.0};
     cudaMemcpyAsync(v, m.sc + 6, 2 * sizeof(double), cudaMemcpyDeviceToHost, st);
     const cudaError_t e = cudaStreamSynchronize(st);
@@ -902,20 +1199,29 @@ struct Run {
   }
 
   // solveMG (multiGrid.f90:165-182): p starts at 0, V-cycles while res > tol_mg.
+  // With p = 0 the residual is q and its ratio 1, so below a tolerance of 1 the
+  // first V-cycle needs no pass to be decided on (for q = 0 it gives p = 0).
   // Each V-cycle is one launch of a CUDA graph captured once per hierarchy
   // (its buffers never move); without a graph the kernels are launched one by one.
   // Adds the V-cycles to *cycles.  A non-finite residual (the FP32 hierarchy
   // overflowed, or a NaN reached it) is a hard error.
   int solve_mg(int *cycles, std::string *err) {
     auto &L = m.lv[0];
-    k_fill<<<nblk_grid(L.n), kMgThreads, 0, st>>>(L.p, L.n, 0.0f);
-    double res = 0.0;
-    int rc = fine_residual(&res, err);
-    int it = 0;
+    double res = 1.0;
+    int rc = TBFP_OK, it = 0;
+    if (m.lv.size() == 1 || !(m.prm.tol_mg < 1.0) || m.prm.max_iter_mg == 0) {
+      k_fill<<<nblk_grid(L.n), kMgThreads, 0, st>>>(L.p, L.n, 0.0f);
+      rc = fine_residual(&res, err);
+    } else {
+      ++it;
+      if (m.zgraph) cudaGraphLaunch(m.zgraph, st);
+      else vcycle(0, true);
+      rc = fine_residual(&res, err);
+    }
     while (rc == TBFP_OK && std::isfinite(res) && it < m.prm.max_iter_mg && res > m.prm.tol_mg) {
       ++it;
       if (m.vgraph) cudaGraphLaunch(m.vgraph, st);
-      else vcycle(0);
+      else vcycle(0, false);
       rc = fine_residual(&res, err);
     }
     *cycles += it;
@@ -927,25 +1233,30 @@ struct Run {
     return TBFP_OK;
   }
 
-  void capture() {
-    if (m.vgraph || m.graph_failed) return;
+  cudaGraphExec_t capture_cycle(bool zero) {
     cudaStream_t cs = nullptr;
     cudaGraph_t gr = nullptr;
+    cudaGraphExec_t ex = nullptr;
     bool ok = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) == cudaSuccess;
     if (ok) ok = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
       Run r{m, cs};
-      r.vcycle(0);
+      r.vcycle(0, zero);
       ok = cudaStreamEndCapture(cs, &gr) == cudaSuccess && gr != nullptr;
     }
-    if (ok) ok = cudaGraphInstantiate(&m.vgraph, gr, 0) == cudaSuccess;
+    if (ok) ok = cudaGraphInstantiate(&ex, gr, 0) == cudaSuccess;
     if (gr) cudaGraphDestroy(gr);
     if (cs) cudaStreamDestroy(cs);
     if (!ok) {
-      m.vgraph = nullptr;
+      ex = nullptr;
       m.graph_failed = true;
       cudaGetLastError();  // clear a capture error; the eager path is used instead
     }
+    return ex;
+  }
+  void capture() {
+    if (!m.vgraph && !m.graph_failed) m.vgraph = capture_cycle(false);
+    if (!m.zgraph && !m.graph_failed) m.zgraph = capture_cycle(true);
   }
 };
 }  // namespace
