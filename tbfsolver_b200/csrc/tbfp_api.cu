@@ -47,6 +47,7 @@ struct tbfp_handle {
   long R = 0;
   int hd_psi = 1, hd_u = 2, hd_rho = 1, hd_st = 1;
   long long wait_cycles = kDefaultWaitCycles;  // bound on each copy wait of the staged correction
+  bool member = false;                         // one of several channels of an ensemble
   Lay Lpsi{}, Lux{}, Luy{}, Luz{}, Lrho{}, Lst[3]{};
   size_t n_psi = 0, n_ux = 0, n_uy = 0, n_uz = 0, n_rho = 0, n_st[3]{};
   int device = 0;
@@ -294,6 +295,10 @@ CorrArgs corr_args(tbfp_handle *h, const double *uxi, const double *uyi, const d
   a.r = dt * alpha;  // momentumEqn.f90:1012
   a.invrho0 = 1.0 / rho0;
   a.wait_cycles = h->wait_cycles;
+  // a caller's own bound on the copy waits asks for the form that has them; small
+  // channels that run side by side load the chip less with it (16 of them: 1.04
+  // ms a call, 1.11 with the kernel form for the small ones)
+  a.staged = h->member || h->wait_cycles != kDefaultWaitCycles;
   return a;
 }
 
@@ -2245,6 +2250,7 @@ int tbfp_ensemble_create(int n, const tbfp_desc *descs, int nstreams, tbfp_ensem
       tbfp_ensemble_destroy(e);
       return set_err(nullptr, rc, m);
     }
+    h->member = n > 1;
     e->h.push_back(h);
     const int T = tri_rows_per_lane(d.ny);
     if (d.precision != TBFP_FP64 || (d.flags & TBFP_FLAG_RESIDUAL) || !ens_supported(d.nx / 2, d.nz, T))

@@ -52,9 +52,16 @@ __device__ __forceinline__ double corr_z(const CorrArgs &a, const GridK &g, int 
   return a.uzi[at(a.Luz, i, j, k)] - a.r * (a.invrho0 * dpr + (invrho - a.invrho0) * dpr0);
 }
 
+// Blocks per SM: with surface tension 80 registers (six blocks) keep a row's ten
+// force loads in flight with the others; 64 (eight) spill them: 0.266 against
+// 0.282 ms on 256x256x128.  (Loaded where they were used, through 64-bit offsets,
+// in chunks of 32 rows: 0.354 ms.)
+constexpr int corr_blocks(bool st) { return st ? 6 : 8; }
+
 template <bool ST>
-__global__ void __launch_bounds__(128, 8) k_correct_div(CorrArgs a, GridK g, unsigned long long *__restrict__ maxdiv) {
-  correct_div_body<ST>(a, g, maxdiv, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x);
+__global__ void __launch_bounds__(128, corr_blocks(ST)) k_correct_div(CorrArgs a, GridK g,
+                                                                      unsigned long long *__restrict__ maxdiv, int jc) {
+  correct_div_body<ST>(a, g, maxdiv, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, jc);
 }
 
 void launch_correct_div(const CorrArgs &ca, bool has_st, const GridK &g, unsigned long long *maxdiv,
@@ -65,9 +72,13 @@ void launch_correct_div(const CorrArgs &ca, bool has_st, const GridK &g, unsigne
         launch_correct_div_tma(ca, g, maxdiv, sms, st))
       return;
   }
-  dim3 grid((g.nx + 127) / 128, (g.ny + kJC - 1) / kJC, g.nz);
-  if (has_st) k_correct_div<true><<<grid, 128, 0, st>>>(ca, g, maxdiv);
-  else k_correct_div<false><<<grid, 128, 0, st>>>(ca, g, maxdiv);
+  // rows per block so that the grid fills whole rounds (96x100x48 with surface
+  // tension: 0.016 ms, in chunks of 32 rows 0.073)
+  const int nbx = (g.nx + 127) / 128;
+  const int jc = march_chunk((long)nbx * g.nz, g.ny, 148L * corr_blocks(has_st), 1);
+  const dim3 grid(nbx, (g.ny + jc - 1) / jc, g.nz);
+  if (has_st) k_correct_div<true><<<grid, 128, 0, st>>>(ca, g, maxdiv, jc);
+  else k_correct_div<false><<<grid, 128, 0, st>>>(ca, g, maxdiv, jc);
 }
 
 // In-place correction: each thread reads and writes only the faces it owns.

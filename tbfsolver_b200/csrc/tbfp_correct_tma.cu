@@ -421,8 +421,15 @@ bool encode_rows(CUtensorMap *m, const double *base, const Lay &Ly, long nk) {
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+constexpr int kMinChunk = 8;
+// Tiles x chunks below which the kernel form is faster: a CTA's march of at least
+// kMinChunk planes takes 21 us however few CTAs there are (32x24x16: 21.2 against
+// 3.7 us; 96x100x48, 78 CTAs: 21.9 against 14.2; 128x128x64, 128 CTAs: 23.0
+// against 25.3; 256x256x128: 152 against 187).
+constexpr int kFewCtas = 100;
+
 // planes per chunk: the chunk count that best fills whole waves of one CTA
-// per SM, counting the extra plane each chunk loads, with at least 8 planes a
+// per SM, counting the extra plane each chunk loads, with at least kMinChunk planes a
 // chunk (small channels run several at once in an ensemble and need not fill
 // the GPU alone)
 int pick_chunk(int tiles, int nz, int sms) {
@@ -430,7 +437,7 @@ int pick_chunk(int tiles, int nz, int sms) {
   double best_eff = -1.0;
   for (int c = 1; c <= 32 && c <= nz; ++c) {
     const int len = (nz + c - 1) / c, chunks = (nz + len - 1) / len;
-    if (len < 8 && len < nz) break;  // a chunk loads one plane more than it corrects
+    if (len < kMinChunk && len < nz) break;  // a chunk loads one plane more than it corrects
     const long ctas = (long)tiles * chunks, waves = (ctas + sms - 1) / sms;
     const double eff = (double)ctas / (double)(waves * sms) * (double)len / (double)(len + 1);
     if (eff > best_eff + 1e-9) {
@@ -453,6 +460,8 @@ cudaError_t prepare_correct_tma_kernel() {
 
 bool launch_correct_div_tma(const CorrArgs &ca, const GridK &g, unsigned long long *maxdiv, int sms,
                             cudaStream_t st) {
+  const int nbx = (g.nx + kCTX - 1) / kCTX, nby = (g.ny + kTY - 1) / kTY;
+  if ((long)nbx * nby * ((g.nz + kMinChunk - 1) / kMinChunk) < kFewCtas && !ca.staged) return false;
   CorrTmaGeom q{};
   if (!box_geom(ca.Lpsi, 0, kCTX + 2, 0, kTY + 2, 1, &q.ps) || !box_geom(ca.Lrho, 0, kCTX + 2, 0, kTY + 2, 1, &q.ir) ||
       !box_geom(ca.Luy, 1, kCTX, 0, kTY + 1, 1, &q.uy) || !box_geom(ca.Luz, 1, kCTX, 1, kTY, 0, &q.uz))
@@ -474,7 +483,6 @@ bool launch_correct_div_tma(const CorrArgs &ca, const GridK &g, unsigned long lo
       !encode_box(&m[3], ca.irho, ca.Lrho, nk_r, q.ir, kTY + 2) || !encode_rows(&m[4], ca.uxi, ca.Lux, nk_u) ||
       !encode_box(&m[5], ca.uyi, ca.Luy, nk_v, q.uy, kTY + 1) || !encode_box(&m[6], ca.uzi, ca.Luz, nk_w, q.uz, kTY))
     return false;
-  const int nbx = (g.nx + kCTX - 1) / kCTX, nby = (g.ny + kTY - 1) / kTY;
   q.nzc = pick_chunk(nbx * nby, g.nz, sms > 0 ? sms : 148);
   const dim3 grid((unsigned)nbx, (unsigned)nby, (unsigned)((g.nz + q.nzc - 1) / q.nzc));
   k_correct_tma<kTY, kNS, kCNT><<<grid, kCNT, (size_t)L.total + 128, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], ca, g, q, maxdiv);

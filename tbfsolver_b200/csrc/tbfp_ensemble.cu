@@ -89,7 +89,7 @@ __device__ __noinline__ void correct_stage(const EnsMember *__restrict__ mp, int
   const EnsMember &m = *mp;
   int bx, by, bz;
   stencil_tile(m.g, kJC, item * 2 + (threadIdx.x >> 7), &bx, &by, &bz);
-  correct_div_body<false, true>(m.ca, m.g, m.maxdiv, bx, by, bz, threadIdx.x & 127);
+  correct_div_body<false, true>(m.ca, m.g, m.maxdiv, bx, by, bz, threadIdx.x & 127, kJC);
 }
 
 __device__ __forceinline__ void run_item(const EnsMember *__restrict__ mp, int stage, int item, unsigned char *sm) {

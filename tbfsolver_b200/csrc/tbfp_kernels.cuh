@@ -75,6 +75,7 @@ struct CorrArgs {
   double r;  // dt*alpha
   double invrho0;
   long long wait_cycles;  // bound on each wait of the TMA-staged correction for its copies (SM cycles)
+  bool staged;            // the staged form however small the grid
 };
 // The max|div u| word of a correction whose copy wait ran out: a NaN with its
 // own payload, above the canonical NaN, so the host tells it from NaN data.

@@ -911,10 +911,10 @@ __device__ __forceinline__ double face_update(double u, double r, double ir0, do
 
 template <bool ST, bool COH = false>
 __device__ __forceinline__ void correct_div_body(CorrArgs a, GridK g, unsigned long long *__restrict__ maxdiv, int bx,
-                                                 int by, int bz, int tx) {
+                                                 int by, int bz, int tx, int jc) {
   const int i = bx * 128 + tx + 1;
   const int k = bz + 1;
-  const int j0 = by * kJC + 1, j1 = min(j0 + kJC - 1, g.ny);
+  const int j0 = by * jc + 1, j1 = min(j0 + jc - 1, g.ny);
   const bool valid = i <= g.nx;
   const int ic = valid ? i : g.nx;  // clamped index keeps every load in bounds
   const int km = (k == 1 && !g.slab) ? g.nz : k - 1;
@@ -941,20 +941,27 @@ __device__ __forceinline__ void correct_div_body(CorrArgs a, GridK g, unsigned l
   const double r = a.r, ir0 = a.invrho0;
   const double idxc = g.idxc1, idzc = g.idzc1;
   const double idx = g.idxf[ic - 1], idz = g.idzf[k - 1];
-  // surface-tension terms of one face (zero without surface tension)
-  auto stf = [&](int c, int ii, int jj, int kk) -> double {
-    if constexpr (ST) {
-      const long q = at(a.Lst[c], ii, jj, kk);
-      return 2.0 * a.stn[c][q] - a.sto[c][q];
-    } else return 0.0;
+  // surface-tension term of one face (zero without surface tension), from the
+  // element offset of the face in its component's array
+  auto stf = [&](int c, int q) -> double {
+    if constexpr (ST) return 2.0 * __ldg(a.stn[c] + q) - __ldg(a.sto[c] + q);
+    else return 0.0;
   };
+  int sx = 0, sy = 0, sz = 0;
+  const int sxj = ST ? (int)a.Lst[0].sj : 0, syj = ST ? (int)a.Lst[1].sj : 0, szj = ST ? (int)a.Lst[2].sj : 0;
+  const int szm = ST ? (km - k) * (int)a.Lst[2].sk : 0;
+  if constexpr (ST) {
+    sx = (int)at(a.Lst[0], ic, j0, k);
+    sy = (int)at(a.Lst[1], ic, j0, k);
+    sz = (int)at(a.Lst[2], ic, j0, k);
+  }
 
   // centre values of the current cell, carried along j
   double psc = ldc<COH>(ps + (op)), pnc = __ldg(pn + (op)), poc = __ldg(po + (op)), irc = ldc<COH>(ir + (oq));
   double uym;
   if (j0 > 1) {
     uym = face_update(__ldg(uyi + (oy - yjs)), r, ir0, irc, ldc<COH>(ir + (oq - rjs)), g.idyc[j0 - 1], psc, ldc<COH>(ps + (op - pjs)), pnc,
-                      __ldg(pn + (op - pjs)), poc, __ldg(po + (op - pjs)), stf(1, ic, j0 - 1, k));
+                      __ldg(pn + (op - pjs)), poc, __ldg(po + (op - pjs)), stf(1, sy - syj));
   } else {
     uym = __ldg(uyi + (oy - yjs));
     if (valid) uyo[oy - yjs] = uym;
@@ -983,17 +990,20 @@ __device__ __forceinline__ void correct_div_body(CorrArgs a, GridK g, unsigned l
     const double psm = ldc<COH>(ps + (op + pm)), pnm = __ldg(pn + (op + pm)), pom = __ldg(po + (op + pm)), irm = ldc<COH>(ir + (oq + qm));
     const double ux_c = __ldg(uxi + (ox)), uy_c = __ldg(uyi + (oy)), uz_c = __ldg(uzi + (oz)), uz_m = __ldg(uzi + (oz + zm));
 
-    const double uxp = face_update(ux_c, r, ir0, irx, irc, idxc, psx, psc, pnx, pnc, pox, poc, stf(0, ic, j, k));
+    const double stx = stf(0, sx), sty = j < g.ny ? stf(1, sy) : 0.0, stz = stf(2, sz), stm = stf(2, sz + szm);
+    const double stw = lead ? stf(0, sx + xo) : 0.0;
+
+    const double uxp = face_update(ux_c, r, ir0, irx, irc, idxc, psx, psc, pnx, pnc, pox, poc, stx);
     const double uxl = lead ? face_update(ux_w, r, ir0, irw1, irw, idxc, psw1, psw, pnw1, pnw, pow1, pow_,
-                                          stf(0, ic + xo, j, k))
+                                          stw)
                             : 0.0;
     const double uxs = __shfl_up_sync(0xffffffffu, uxp, 1);
     const double uxm = lead ? uxl : uxs;
     const double uyp = (j < g.ny) ? face_update(uy_c, r, ir0, iry, irc, g.idyc[j], psy, psc, pny, pnc, poy, poc,
-                                                stf(1, ic, j, k))
+                                                sty)
                                   : uy_c;
-    const double uzp = face_update(uz_c, r, ir0, irz, irc, idzc, psz, psc, pnz, pnc, poz, poc, stf(2, ic, j, k));
-    const double uzq = face_update(uz_m, r, ir0, irc, irm, idzc, psc, psm, pnc, pnm, poc, pom, stf(2, ic, j, km));
+    const double uzp = face_update(uz_c, r, ir0, irz, irc, idzc, psz, psc, pnz, pnc, poz, poc, stz);
+    const double uzq = face_update(uz_m, r, ir0, irc, irm, idzc, psc, psm, pnc, pnm, poc, pom, stm);
     if (valid) {
       uxo[ox] = uxp;
       if (i == g.nx) uxo[ox - ic] = uxp;  // ux(0, j, k)
@@ -1015,6 +1025,9 @@ __device__ __forceinline__ void correct_div_body(CorrArgs a, GridK g, unsigned l
     ox += xjs;
     oy += yjs;
     oz += zjs;
+    sx += sxj;
+    sy += syj;
+    sz += szj;
   }
   block_max_atomic(vmax, maxdiv);
 }

@@ -369,3 +369,70 @@ def test_errors_are_raised_not_hidden():
         with pytest.raises(TbfpError):
             eqn.projection(f, f, f, f, u, dt=-1.0, alpha=1.0)
         eqn.close()
+
+
+@pytest.mark.parametrize("dims", [(8, 5, 4), (32, 24, 16), (96, 100, 48), (256, 37, 16), (128, 96, 64)])
+def test_both_forms_of_the_correction_give_the_same_velocity(dims):
+    """Grids too small to fill the staged correction take the kernel form; a wait
+    limit of the caller's own keeps the staged one.  Both evaluate every face in
+    the same order: the same bits, rows per block 1 and more, one and two x tiles,
+    partial tiles."""
+    nx, ny, nz = dims
+    spec = synth.small_spec(nx, ny, nz, nbubbles=2, radius=0.3, rhog=0.05)
+    inp = synth.make_inputs(spec, seed=nx + ny, device="cuda")
+    rng = np.random.default_rng(nz)
+    for f in (inp.psi_n, inp.psi_nm1):
+        a = rng.standard_normal(f.a.shape)
+        f.a.copy_(torch.from_numpy(a))
+        synth.update_boundaries_cl(f.a, 1, nx, ny, nz)
+    got = []
+    eqn = PoissonEqn(inp.grid, spec.rhol, spec.rhog)
+    try:
+        for limit in (4_000_000_000, 5_000_000_000):  # the default, and another
+            eqn.solver.set_wait_limit(limit)
+            psi = Field.like(inp.psi_n, torch.zeros_like(inp.psi_n.a))
+            uo = VField(*[Field.like(f, torch.zeros_like(f.a)) for f in inp.u.components()])
+            torch.cuda.synchronize()
+            st = eqn.projection(psi, inp.psi_n, inp.psi_nm1, inp.rho, inp.u, inp.dt, inp.alpha, u_out=uo)
+            got.append(([f.a for f in uo.components()], st.max_div))
+    finally:
+        eqn.close()
+    for a, b in zip(*[g[0] for g in got]):
+        assert torch.equal(a, b)
+    assert got[0][1] == got[1][1]
+
+
+@pytest.mark.parametrize("dims", [(8, 5, 4), (96, 13, 48), (256, 37, 16)])
+def test_surface_tension_correction_chunks_match_the_oracle(dims):
+    """Rows per block from one to all of them, with remainders, on random force
+    fields at both levels."""
+    nx, ny, nz = dims
+    spec = synth.small_spec(nx, ny, nz, nbubbles=2, radius=0.3, rhog=0.05)
+    inp = synth.make_inputs(spec, seed=ny)
+    g, rng = inp.grid, np.random.default_rng(nx)
+    st = []
+    for _ in range(2):
+        fs = [O.FField(k, 1, nx, ny, nz, rng.standard_normal(Field(k, 1, nx, ny, nz).a.shape)) for k in ("sx", "sy", "sz")]
+        for f in fs:
+            f.a[...] *= 0.01
+        fs[0].a[:, :, 1] = fs[0].a[:, :, -2]          # periodic duplicate faces
+        fs[2].a[1] = fs[2].a[-2]
+        fs[1].a[:, 1, :] = fs[1].a[:, -2, :] = 0.0    # no force on the wall faces
+        st.append(fs)
+    ref = O.projection(mesh_of(g), *[to_oracle(f, g) for f in (inp.u.ux, inp.u.uy, inp.u.uz, inp.rho, inp.psi_n,
+                                                              inp.psi_nm1)], inp.dt, inp.alpha, inp.rho0, *st)
+    cu = lambda f: Field(f.kind, f.hd, nx, ny, nz, torch.as_tensor(f.a).cuda())  # noqa: E731
+    eqn = PoissonEqn(g, spec.rhol, spec.rhog)
+    try:
+        u = VField(*[cu(f) for f in inp.u.components()])
+        uo = VField(*[Field.like(f, torch.zeros_like(f.a)) for f in u.components()])
+        psi = cu(inp.psi_n)
+        torch.cuda.synchronize()
+        eqn.projection(psi, cu(inp.psi_n), cu(inp.psi_nm1), cu(inp.rho), u, inp.dt, inp.alpha,
+                       [cu(f) for f in st[0]], [cu(f) for f in st[1]], u_out=uo)
+        assert rel_linf(psi.a.cpu().numpy(), ref.psi.a) < TOL_P
+        boxes = [(0, nx, 1, ny, 1, nz), (1, nx, 0, ny, 1, nz), (1, nx, 1, ny, 0, nz)]
+        for f, r, b in zip(uo.components(), (ref.ux, ref.uy, ref.uz), boxes):
+            assert rel_linf(Field.like(f, f.a.cpu().numpy()).v(*b), r.v(*b)) < TOL_P
+    finally:
+        eqn.close()
