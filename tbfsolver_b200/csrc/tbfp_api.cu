@@ -570,9 +570,8 @@ int device_projection(tbfp_handle *h, const double *uxi, const double *uyi, cons
     if (timing) cudaEventRecord(h->evs[i], s);
   };
   TBFP_CK(h, cudaEventRecord(h->ev0, s));
-  TBFP_CK(h, cudaMemsetAsync(h->d_maxdiv, 0, sizeof(unsigned long long), s));
   mark(0);
-  launch_recip(rho, h->d_irho, (long)h->n_rho, s);
+  launch_recip(rho, h->d_irho, (long)h->n_rho, s, h->d_maxdiv);
   mark(1);
   RhsArgs ra = rhs_args(h, uxi, uyi, uzi, psi_n, psi_nm1, st_n, st_nm1, dt, alpha, rho0);
   int iters = 1, solve_rc = TBFP_OK;

@@ -290,7 +290,9 @@ void set_global_error(const std::string &msg);
 // Kernel launchers.  The x launchers take twx (fft_unit_twiddles(nx)) and tpx
 // (fft_pass_twiddles(nx/2)); the z launcher takes tpz (fft_pass_twiddles(nz)).
 cudaError_t prepare_kernels();  // raises the shared-memory limits; once per device
-void launch_recip(const double *rho, double *irho, long n, cudaStream_t st);
+// zero: a word that the same launch clears (the projection's max|div u|, which a
+// memset of its own took 1.5 us and a launch gap to clear), or NULL
+void launch_recip(const double *rho, double *irho, long n, cudaStream_t st, unsigned long long *zero = nullptr);
 void launch_fftx_fwd_from_s(const double *s, Lay Ls, const GridK &g, const double2 *twx, const double2 *tpx,
                             double2 *spec, cudaStream_t st);
 void launch_rhs(const RhsArgs &ra, bool has_st, const GridK &g, double *s, Lay Ls, cudaStream_t st);

@@ -17,14 +17,18 @@ namespace tbfp {
 // ---------------------------------------------------------------------------
 // 1/rho over the whole (halo-inclusive) density array.
 // ---------------------------------------------------------------------------
-__global__ void k_recip(const double *__restrict__ rho, double *__restrict__ irho, long n) {
+__global__ void k_recip(const double *__restrict__ rho, double *__restrict__ irho, long n,
+                        unsigned long long *__restrict__ zero) {
+  if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0ull;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
     irho[t] = 1.0 / rho[t];
 }
 
 // The same with 16-byte accesses, two in flight per thread (both arrays
 // 16-byte aligned; the odd last element, if any, by the scalar kernel's rule).
-__global__ void k_recip2(const double2 *__restrict__ rho, double2 *__restrict__ irho, long n2) {
+__global__ void k_recip2(const double2 *__restrict__ rho, double2 *__restrict__ irho, long n2,
+                         unsigned long long *__restrict__ zero) {
+  if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0ull;
   const long stride = (long)gridDim.x * blockDim.x;
   long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   for (; t + stride < n2; t += 2 * stride) {
@@ -38,19 +42,19 @@ __global__ void k_recip2(const double2 *__restrict__ rho, double2 *__restrict__ 
   }
 }
 
-void launch_recip(const double *rho, double *irho, long n, cudaStream_t st) {
+void launch_recip(const double *rho, double *irho, long n, cudaStream_t st, unsigned long long *zero) {
   if (((reinterpret_cast<uintptr_t>(rho) | reinterpret_cast<uintptr_t>(irho)) & 15) == 0 && n >= 2) {
     const long n2 = n / 2;
     long blocks = (n2 + 511) / 512;
     if (blocks > 148 * 8) blocks = 148 * 8;
     k_recip2<<<(unsigned)blocks, 256, 0, st>>>(reinterpret_cast<const double2 *>(rho),
-                                              reinterpret_cast<double2 *>(irho), n2);
-    if (n & 1) k_recip<<<1, 32, 0, st>>>(rho + (n - 1), irho + (n - 1), 1);
+                                              reinterpret_cast<double2 *>(irho), n2, zero);
+    if (n & 1) k_recip<<<1, 32, 0, st>>>(rho + (n - 1), irho + (n - 1), 1, nullptr);
     return;
   }
   int blocks = (int)((n + 255) / 256);
   if (blocks > 148 * 16) blocks = 148 * 16;
-  k_recip<<<blocks, 256, 0, st>>>(rho, irho, n);
+  k_recip<<<blocks, 256, 0, st>>>(rho, irho, n, zero);
 }
 
 // ---------------------------------------------------------------------------
