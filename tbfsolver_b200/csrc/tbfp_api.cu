@@ -578,7 +578,12 @@ int device_projection(tbfp_handle *h, const double *uxi, const double *uyi, cons
   double rel = -1.0;
   const bool read = stats != nullptr || !(h->flags & TBFP_FLAG_ASYNC);
   if (h->precision == TBFP_FP64 && !(h->flags & TBFP_FLAG_RESIDUAL)) {
-    launch_rhs_fftx(ra, st, h->g, h->d_twx, h->d_tpx, h->d_spec, s);  // s stays on chip
+    if (h->g.M < kRhsFftxMaxM) {
+      launch_rhs_fftx(ra, st, h->g, h->d_twx, h->d_tpx, h->d_spec, s);  // s stays on chip
+    } else {
+      launch_rhs(ra, st, h->g, h->d_s, h->Lpsi, s);
+      launch_fftx_fwd_from_s(h->d_s, h->Lpsi, h->g, h->d_twx, h->d_tpx, h->d_spec, s);
+    }
     mark(2);
     launch_fftz(h->d_spec, h->g, h->d_tpz, false, s);
     mark(3);

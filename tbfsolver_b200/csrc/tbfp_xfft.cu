@@ -353,7 +353,7 @@ void launch_rhs(const RhsArgs &ra, bool has_st, const GridK &g, double *s, Lay L
 // post-processing and the transposed store are those of k_fftx_fwd.
 // ---------------------------------------------------------------------------
 template <int M, bool ST>
-__global__ void __launch_bounds__(kNT, (M >= 384 ? 2 : 3))
+__global__ void __launch_bounds__(kNT, 3)
     k_rhs_fftx(RhsArgs a, GridK g, const double2 *__restrict__ twx, const double2 *__restrict__ tpx,
                double2 *__restrict__ spec) {
   using V = double2;
@@ -504,9 +504,9 @@ void launch_rhs_fftx(const RhsArgs &ra, bool has_st, const GridK &g, const doubl
   switch (g.M) {
 #define TBFP_CASE(L) \
   case L: launch_rhs_fftx_n<L>(ra, has_st, g, twx, tpx, spec, st); break;
-    TBFP_FFT_LENGTHS(TBFP_CASE)
+    TBFP_RHS_FFTX_LENGTHS(TBFP_CASE)
 #undef TBFP_CASE
-    default: break;  // lengths are validated by tbfp_create
+    default: break;  // the caller takes this form below kRhsFftxMaxM only
   }
 }
 
@@ -721,10 +721,13 @@ cudaError_t prepare_xfft_kernels() {
   set((const void *)k_fftx_fwd<float2, L, 1>, fftx_smem_bytes(L, 8));        \
   set((const void *)k_fftx_inv<double2, L, false>, fftx_smem_bytes(L, 16));  \
   set((const void *)k_fftx_inv<float2, L, false>, fftx_smem_bytes(L, 8));    \
-  set((const void *)k_fftx_inv<float2, L, true>, fftx_smem_bytes(L, 8));     \
-  set((const void *)k_rhs_fftx<L, false>, fftx_smem_bytes(L, 16));           \
-  set((const void *)k_rhs_fftx<L, true>, fftx_smem_bytes(L, 16));
+  set((const void *)k_fftx_inv<float2, L, true>, fftx_smem_bytes(L, 8));
   TBFP_FFT_LENGTHS(TBFP_CASE)
+#undef TBFP_CASE
+#define TBFP_CASE(L)                                               \
+  set((const void *)k_rhs_fftx<L, false>, fftx_smem_bytes(L, 16)); \
+  set((const void *)k_rhs_fftx<L, true>, fftx_smem_bytes(L, 16));
+  TBFP_RHS_FFTX_LENGTHS(TBFP_CASE)
 #undef TBFP_CASE
   set((const void *)k_fftx_inv_pf<128>, fftx_inv_pf_smem_bytes<128>());
   set((const void *)k_fftx_inv_pf<256>, fftx_inv_pf_smem_bytes<256>());
