@@ -183,8 +183,9 @@ __device__ __forceinline__ double face_pos(const StGrid &g, int d, int q) {
 // A warp takes 32 listed cells.  The normal and the curvature formula run one
 // cell per lane; in between the cells' height columns (nine per cell) are dealt
 // out to the lanes, whatever cell they belong to, 32 at a time, and leave their
-// interface positions in shared memory.  A cell without a valid first direction
-// takes another round with its second and third.  The 13 class bytes of a column are
+// interface positions in shared memory; the eight around a cell's own column wait
+// until that one has proved valid.  A cell without a valid first direction takes
+// another round with its second and third.  The 13 class bytes of a column are
 // loaded at once, so its two ends are bit scans and not walks of dependent loads.
 // Sums are taken in the order of the restatement, so a rounding cannot turn a
 // decision.  Bound: instructions of the columns and L1 misses on c's rows; one
@@ -253,86 +254,96 @@ __global__ void __launch_bounds__(32 * kCurvWarps, kCurvBlocks) k_st_curvature(c
     bool found = !live;
     double kv = 0.0;
     for (int r = 0; r < 3; ++r) {
-      const unsigned pend = __ballot_sync(all, !found);
-      if (pend == 0) break;
-      const int ncol = 9 * __popc(pend);
+      if (!__any_sync(all, !found)) break;
       bad[wib][lane] = 0;
-      if (!found) slot[wib][__popc(pend & ((1u << lane) - 1u))] = lane;
       __syncwarp();
-      for (int q = lane; q < ((ncol + 31) & ~31); q += 32) {
-        const bool have = q < ncol;
-        const int own = have ? slot[wib][q / 9] : 0, col = q % 9;  // the cell's lane, its column
+      int ncol = 0;  // columns of the passes after the first
+      for (int pass = 0; pass == 0 || 32 * (pass - 1) < ncol; ++pass) {
+        // the first pass walks every open cell's own column, the others the eight
+        // around it of the cells where that one is valid
+        const int q = 32 * (pass - 1) + lane, e = q & 7;
+        const bool have = pass == 0 ? !found : q < ncol;
+        const int own = pass == 0 ? lane : (have ? slot[wib][q >> 3] : 0), col = pass == 0 ? 4 : e + (e >= 4);
         const int oi = __shfl_sync(all, i, own), oj = __shfl_sync(all, j, own), ok_ = __shfl_sync(all, k, own);
         const int od = __shfl_sync(all, ord, own) >> (2 * r) & 3, os = __shfl_sync(all, sgn, own);
-        if (!have) continue;
-        const int d = od, s = os >> d & 1 ? -1 : 1;
-        // the column's start cell, one step across the direction
-        const int da = col / 3 - 1, db = col % 3 - 1;
-        int ci = oi + (d != 0 ? da : 0), cj = oj + (d == 0 ? da : (d == 2 ? db : 0)), ck = ok_ + (d != 2 ? db : 0);
-        bool ok = cj >= 0 && cj < g.ny;
-        ci = ci < 0 ? ci + g.nx : (ci >= g.nx ? ci - g.nx : ci);
-        cj = clampj(g, cj);
-        ck = ck < 0 ? ck + g.nz : (ck >= g.nz ? ck - g.nz : ck);
-        const int q0 = d == 0 ? ci : (d == 1 ? cj : ck), nd = d == 0 ? g.nx : (d == 1 ? g.ny : g.nz);
-        const int dd = d == 0 ? 1 : (d == 1 ? g.nx : g.nx * g.ny);
-        const long cd = d == 0 ? 1 : (d == 1 ? Lc.sj : Lc.sk);
-        const unsigned char *fr = fl + dix(g, ci, cj, ck);
-        const double *cr = c + at(Lc, ci + 1, cj + 1, ck + 1);
-        // class nibbles, the cell at -kStColumn steps (away from the full phase) lowest
-        unsigned long long w = 0;
-        const bool inside = q0 >= kStColumn && q0 + kStColumn < nd;
-        if (inside) {
-          const unsigned char *f0 = fr - (long)(s * kStColumn) * dd;
-          const long sd = (long)s * dd;
-          unsigned lo = 0, hi = 0;
-#pragma unroll
-          for (int u = 0; u <= 2 * kStColumn; ++u) {
-            if (u < 8) lo |= (unsigned)f0[u * sd] << (4 * u);
-            else hi |= (unsigned)f0[u * sd] << (4 * (u - 8));
-          }
-          w = (unsigned long long)hi << 32 | lo;
-        } else {  // near a wall, where columns stop, or across a periodic boundary
-#pragma unroll 1
-          for (int u = 0; u <= 2 * kStColumn; ++u) {
-            int x = q0 + s * (u - kStColumn);
-            unsigned f = kMixed;  // beyond a wall: no end of the column
-            if (d != 1 || (x >= 0 && x < nd)) {
-              x = wrapn(x, nd);
-              f = fr[(long)(x - q0) * dd];
+        if (have) {
+          const int d = od, s = os >> d & 1 ? -1 : 1;
+          // the column's start cell, one step across the direction
+          const int da = col / 3 - 1, db = col % 3 - 1;
+          int ci = oi + (d != 0 ? da : 0), cj = oj + (d == 0 ? da : (d == 2 ? db : 0)), ck = ok_ + (d != 2 ? db : 0);
+          bool ok = cj >= 0 && cj < g.ny;
+          ci = ci < 0 ? ci + g.nx : (ci >= g.nx ? ci - g.nx : ci);
+          cj = clampj(g, cj);
+          ck = ck < 0 ? ck + g.nz : (ck >= g.nz ? ck - g.nz : ck);
+          const int q0 = d == 0 ? ci : (d == 1 ? cj : ck), nd = d == 0 ? g.nx : (d == 1 ? g.ny : g.nz);
+          const int dd = d == 0 ? 1 : (d == 1 ? g.nx : g.nx * g.ny);
+          const long cd = d == 0 ? 1 : (d == 1 ? Lc.sj : Lc.sk);
+          const unsigned char *fr = fl + dix(g, ci, cj, ck);
+          const double *cr = c + at(Lc, ci + 1, cj + 1, ck + 1);
+          // class nibbles, the cell at -kStColumn steps (away from the full phase) lowest
+          unsigned long long w = 0;
+          const bool inside = q0 >= kStColumn && q0 + kStColumn < nd;
+          if (inside) {
+            const unsigned char *f0 = fr - (long)(s * kStColumn) * dd;
+            const long sd = (long)s * dd;
+            unsigned lo = 0, hi = 0;
+  #pragma unroll
+            for (int u = 0; u <= 2 * kStColumn; ++u) {
+              if (u < 8) lo |= (unsigned)f0[u * sd] << (4 * u);
+              else hi |= (unsigned)f0[u * sd] << (4 * (u - 8));
             }
-            w |= (unsigned long long)f << (4 * u);
-          }
-        }
-        const unsigned long long ones = 0x1111111111111ull;
-        // bit 4u: the cell u is full / empty
-        const unsigned long long wf = (w >> 1 & ones) >> (4 * kStColumn);
-        const unsigned long long we = (~(w | w >> 1) & ones) << (63 - 4 * kStColumn);
-        const int tf = wf ? (__ffsll((long long)wf) - 1) >> 2 : -1;  // steps to the first full cell
-        const int te = we ? __clzll((long long)we) >> 2 : -1;        // and back to the first empty one
-        ok = ok && tf >= 0 && te >= 0;
-        double f = 0.0;
-        if (ok) {
-          double hs = 0.0;
-          if (inside && (w & (kPromoted * ones)) == 0) {
-            const double *pc = cr - (long)(s * te) * cd;
-            const double wd = d == 0 ? g.dx : g.dz;
-            int x = q0 - s * te;
-            for (int u = te + tf; u >= 0; --u, pc += s * cd, x += s)
-              hs = __dadd_rn(hs, __dmul_rn(*pc, d == 1 ? g.dyf[x] : wd));
-          } else {
-            for (int u = -te; u <= tf; ++u) {
-              int x = q0 + s * u;
-              if (d != 1) x = wrapn(x, nd);
-              const double v = (w >> (4 * (u + kStColumn)) & kPromoted) ? 1.0 - 2.0 * eps : cr[(x - q0) * cd];
-              hs = __dadd_rn(hs, __dmul_rn(v, d == 0 ? g.dx : (d == 2 ? g.dz : g.dyf[x])));
+            w = (unsigned long long)hi << 32 | lo;
+          } else {  // near a wall, where columns stop, or across a periodic boundary
+  #pragma unroll 1
+            for (int u = 0; u <= 2 * kStColumn; ++u) {
+              int x = q0 + s * (u - kStColumn);
+              unsigned f = kMixed;  // beyond a wall: no end of the column
+              if (d != 1 || (x >= 0 && x < nd)) {
+                x = wrapn(x, nd);
+                f = fr[(long)(x - q0) * dd];
+              }
+              w |= (unsigned long long)f << (4 * u);
             }
           }
-          const int qf = q0 + s * tf;  // not wrapped: the nine columns share one frame
-          const double xf = face_pos(g, d, s > 0 ? qf + 1 : qf);
-          f = s > 0 ? __dsub_rn(xf, hs) : __dadd_rn(xf, hs);
+          const unsigned long long ones = 0x1111111111111ull;
+          // bit 4u: the cell u is full / empty
+          const unsigned long long wf = (w >> 1 & ones) >> (4 * kStColumn);
+          const unsigned long long we = (~(w | w >> 1) & ones) << (63 - 4 * kStColumn);
+          const int tf = wf ? (__ffsll((long long)wf) - 1) >> 2 : -1;  // steps to the first full cell
+          const int te = we ? __clzll((long long)we) >> 2 : -1;        // and back to the first empty one
+          ok = ok && tf >= 0 && te >= 0;
+          double f = 0.0;
+          if (ok) {
+            double hs = 0.0;
+            if (inside && (w & (kPromoted * ones)) == 0) {
+              const double *pc = cr - (long)(s * te) * cd;
+              const double wd = d == 0 ? g.dx : g.dz;
+              int x = q0 - s * te;
+              for (int u = te + tf; u >= 0; --u, pc += s * cd, x += s)
+                hs = __dadd_rn(hs, __dmul_rn(*pc, d == 1 ? g.dyf[x] : wd));
+            } else {
+              for (int u = -te; u <= tf; ++u) {
+                int x = q0 + s * u;
+                if (d != 1) x = wrapn(x, nd);
+                const double v = (w >> (4 * (u + kStColumn)) & kPromoted) ? 1.0 - 2.0 * eps : cr[(x - q0) * cd];
+                hs = __dadd_rn(hs, __dmul_rn(v, d == 0 ? g.dx : (d == 2 ? g.dz : g.dyf[x])));
+              }
+            }
+            const int qf = q0 + s * tf;  // not wrapped: the nine columns share one frame
+            const double xf = face_pos(g, d, s > 0 ? qf + 1 : qf);
+            f = s > 0 ? __dsub_rn(xf, hs) : __dadd_rn(xf, hs);
+          }
+          Fs[wib][own][col] = f;
+          if (!ok) bad[wib][own] = 1;
         }
-        Fs[wib][own][col] = f;
-        if (!ok) bad[wib][own] = 1;
+        if (pass == 0) {
+          __syncwarp();
+          const bool open = !found && !bad[wib][lane];
+          const unsigned m = __ballot_sync(all, open);
+          if (open) slot[wib][__popc(m & ((1u << lane) - 1u))] = lane;
+          ncol = 8 * __popc(m);
+          __syncwarp();
+        }
       }
       __syncwarp();
       if (!found && !bad[wib][lane]) {
