@@ -503,7 +503,7 @@ __global__ void k_coarse_apply(MgLev L, const double *__restrict__ M, int n1, co
 // ---------------------------------------------------------------------------
 constexpr int kMgMaxLevels = 16, kTailThreads = 1024;
 constexpr size_t kTailSmem = 64 * 1024;
-constexpr int kTailCoarse = 512;  // unknowns of the coarsest system whose inverse one SM applies (2 MB of it)
+constexpr int kTailCoarse = 320;  // unknowns of the coarsest system whose inverse (0.8 MB) one SM applies
 struct MgTail {
   int n;  // levels, the last one the coarsest
   int n_pre, n_post;
@@ -1050,13 +1050,13 @@ int MgSolver::init(const tbfp_mg_params &prm, int nx, int ny, int nz, const doub
     G.py = L.tab + o[13];
     G.pz = L.tab + o[14];
   }
-  // the coarse levels small enough for one SM (k_mg_tail), if the coarsest system is
+  // the coarse levels small enough for one SM (k_mg_tail), if the coarsest system
+  // is, and with at least one level to smooth: many SMs apply the inverse faster
   m.tail = prm.n_levels;
-  if (m.n1 <= kTailCoarse)
-    for (int l = prm.n_levels - 1; l >= 1; --l) {
-    size_t b = 8 * (size_t)m.lv.back().n;
-    for (int r = l; r + 1 < prm.n_levels; ++r) b += 12 * (size_t)m.lv[r].n;
-    if (b > kTailSmem || prm.n_levels - l > kMgMaxLevels) break;
+  size_t tb = 8 * (size_t)m.lv.back().n;
+  for (int l = prm.n_levels - 2; l >= 1 && m.n1 <= kTailCoarse && prm.n_levels - l <= kMgMaxLevels; --l) {
+    tb += 12 * (size_t)m.lv[l].n;
+    if (tb > kTailSmem) break;
     m.tail = l;
   }
   ck(cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));

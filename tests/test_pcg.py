@@ -148,12 +148,13 @@ def test_mg_projection_matches_the_oracle():
 
 @pytest.mark.parametrize("dims, levels, sweeps, cycles", [((96, 24, 16), 3, (2, 2), 1), ((64, 30, 8), 2, (1, 2), 2),
                                                           ((32, 8, 8), 2, (0, 1), 1), ((32, 16, 12), 3, (1, 0), 2),
-                                                          ((128, 12, 64), 3, (2, 1), 1), ((128, 48, 32), 4, (2, 2), 2)])
+                                                          ((128, 12, 64), 3, (2, 1), 1), ((128, 48, 32), 4, (2, 2), 2),
+                                                          ((16, 12, 8), 1, (2, 2), 1), ((32, 16, 16), 2, (2, 2), 1)])
 def test_v_cycles_match_the_oracle(dims, levels, sweeps, cycles):
     """One PCG iteration with a fixed number of V-cycles against the FP64 oracle:
     tiles cut in x and y and filled exactly, marches of one and several chunks,
-    odd numbers of smoothing iterations, none before or after, coarse ends of one
-    to three levels.  (A uniform grid: on a stretched one the library's coarse
+    odd numbers of smoothing iterations, none before or after, coarse ends of no
+    to three levels, a single level.  (A uniform grid: on a stretched one the library's coarse
     ghost centroids are mirror images where the oracle evaluates the grid formula.)
     Bar: the cycles run in FP32 (6e-8 a rounding, some 100 of them behind one
     another), 2e-5 of the largest pressure."""
