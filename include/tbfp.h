@@ -435,8 +435,10 @@ int tbfp_ensemble_get_mode(const tbfp_ensemble *e, int *mode, int *param, float 
    shared memory (the FP64 out-of-place correction of tbfp_projection[_dev] and of each ensemble
    member), in SM clock cycles; default 4e9 (about 2 s), 0: a copy not complete at the first look
    counts as late.  A wait that runs out ends the kernel after its copies in flight have landed:
-   the call returns TBFP_ETIMEOUT and the handle stays usable.  No counterpart in the reference
-   (its loops run on the host and cannot wait on a copy engine). */
+   the call returns TBFP_ETIMEOUT and the handle stays usable.  With the default bound, grids too
+   small to fill the staged form run one that copies nothing (the same results, bit for bit); any
+   other bound keeps the staged form.  No counterpart in the reference (its loops run on the host
+   and cannot wait on a copy engine). */
 int tbfp_set_wait_limit(tbfp_handle *h, long long cycles);
 /* Bound on each dependency wait of the persistent kernel, in polls of about 0.1 us (default 1e7,
    about a second).  A wait that runs out stops the launch: the call returns TBFP_ETIMEOUT. */
