@@ -472,6 +472,14 @@ __global__ void __launch_bounds__(256) k_gj_update(double *__restrict__ M, int n
   }
 }
 
+// Right-hand side -V s of cell t on the coarsest level, in FP64: a product of four
+// FP32 factors whose scale is the caller's (cell volume times source) can leave the
+// FP32 range although s and the pressure are well inside it.
+__device__ __forceinline__ double coarse_rhs(const MgLev &L, int t, float s) {
+  const int r = t / L.nx, k = r / L.ny, i = t - r * L.nx, j = r - k * L.ny;
+  return -((double)L.vx[i] * (double)L.vy[j] * (double)L.vz[k]) * (double)s;
+}
+
 // p = K^-1 (-V s) on the coarsest level (the Lagrange row's right-hand side is
 // 0); the inverse is stored in the reordered basis.
 __global__ void k_coarse_apply(MgLev L, const double *__restrict__ M, int n1, const float *__restrict__ s,
@@ -481,11 +489,7 @@ __global__ void k_coarse_apply(MgLev L, const double *__restrict__ M, int n1, co
   if (warp >= n) return;
   const long row = (long)coarse_perm(warp, n) * ld + n1;
   double acc = 0.0;
-  for (int c = lane; c < n; c += 32) {
-    const int i = c % L.nx, j = (c / L.nx) % L.ny, k = c / (L.nx * L.ny);
-    const double V = (double)L.vx[i] * (double)L.vy[j] * (double)L.vz[k];
-    acc += M[row + coarse_perm(c, n)] * (-V * (double)s[c]);
-  }
+  for (int c = lane; c < n; c += 32) acc += M[row + coarse_perm(c, n)] * coarse_rhs(L, c, s[c]);
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) p[warp] = (float)acc;
 }
@@ -595,19 +599,16 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_consta
     }
     __syncthreads();
   }
-  {  // p = K^-1 (-V q) on the coarsest level (k_coarse_apply)
-    const MgLev &L = T.L[last];
+  {  // p = K^-1 (-V q) on the coarsest level, as k_coarse_apply
+    __shared__ double rhs[kTailCoarse];
     const int n = T.n1 - 1, ld = 2 * T.n1, lane = tid & 31;
-    for (int t = tid; t < n; t += kTailThreads) {
-      const int r = t / L.nx, k = r / L.ny;
-      q[last][t] *= -(L.vx[t - r * L.nx] * L.vy[r - k * L.ny] * L.vz[k]);
-    }
+    for (int t = tid; t < n; t += kTailThreads) rhs[t] = coarse_rhs(T.L[last], t, q[last][t]);
     __syncthreads();
     for (int r = tid >> 5; r < n; r += kTailThreads / 32) {
       const double *row = T.M + (long)coarse_perm(r, n) * ld + T.n1;
       double acc = 0.0;
 #pragma unroll 4
-      for (int c = lane; c < n; c += 32) acc += row[coarse_perm(c, n)] * (double)q[last][c];
+      for (int c = lane; c < n; c += 32) acc += row[coarse_perm(c, n)] * rhs[c];
       for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
       if (lane == 0) p[last][r] = (float)acc;
     }

@@ -168,3 +168,27 @@ def test_v_cycles_match_the_oracle(dims, levels, sweeps, cycles):
     assert st.iterations == 1
     a, b = O.FField("cl", 1, nx, ny, nz, psi).interior(), ref.interior()
     assert rel_linf(a - a.mean(), b - b.mean()) < 2e-5
+
+
+def test_coarse_system_keeps_the_scale_of_a_small_domain():
+    """Lengths of 1e-5 and a source of 1e-28: the pressure (2e-36) is well inside the FP32 range, the product of
+    cell volume and source on the coarsest level (3e-45 at most) is not, and the coarse end of the cycle holds it in
+    FP64.  One PCG iteration of one V-cycle against the FP64 oracle; bar as above, 2e-5 of the largest pressure
+    (with the product in FP32 the error is 1.4e-2)."""
+    nx, ny, nz = 32, 16, 16
+    g = Grid(nx, ny, nz, 2e-5, 1e-5, 1e-5)
+    m = mesh_of(g)
+    rng = np.random.default_rng(8)
+    j, i = np.arange(ny)[None, :, None] + 0.5, np.arange(nx)[None, None, :] + 0.5
+    q = np.cos(np.pi * j / ny) + np.sin(2 * np.pi * i / nx) + 0.1 * rng.standard_normal((nz, ny, nx))
+    q = 1e-28 * (q - q.mean())
+    beta = O.FField("cl", 1, nx, ny, nz)
+    beta.v(1, nx, 1, ny, 1, nz)[...] = 1e-3 * (0.5 + rng.random((nz, ny, nx)))
+    O.update_boundaries_cl_channel(beta)
+    kw = dict(n_pre=2, n_post=2, tol_mg=1e-9, max_iter_mg=1, tol_pcg=1e-10, max_iter_pcg=1)
+    ref = O.FField("cl", 1, nx, ny, nz)
+    O.MGOracle(m, n_levels=3, **kw).solve_pcg(ref, beta, q)
+    st, psi = _gpu_pcg(g, q, beta, 3, **kw)
+    assert st.iterations == 1
+    a, b = O.FField("cl", 1, nx, ny, nz, psi).interior(), ref.interior()
+    assert rel_linf(a - a.mean(), b - b.mean()) < 2e-5
