@@ -1180,8 +1180,8 @@ struct Run {
   }
 
   // ||q - L p|| / ||q|| at the finest level (computeResiduals' res) into *res;
-  // a CUDA error returns TBFP_ECUDA with its text in *err.
-  int fine_residual(double *res, std::string *err) {
+  // a CUDA error returns TBFP_ECUDA with its text in *err.  *q_zero: whether q = 0.
+  int fine_residual(double *res, std::string *err, bool *q_zero = nullptr) {
     auto &L = m.lv[0];
     cudaMemsetAsync(m.sc + 6, 0, 2 * sizeof(double), st);
     if (m.lv.size() > 1)
@@ -1196,12 +1196,14 @@ struct Run {
       return TBFP_ECUDA;
     }
     *res = std::sqrt(v[0]) / (std::sqrt(v[1]) + 1e-300);
+    if (q_zero) *q_zero = v[1] == 0.0;
     return TBFP_OK;
   }
 
   // solveMG (multiGrid.f90:165-182): p starts at 0, V-cycles while res > tol_mg.
   // With p = 0 the residual is q and its ratio 1, so below a tolerance of 1 the
-  // first V-cycle needs no pass to be decided on (for q = 0 it gives p = 0).
+  // first V-cycle needs no pass to be decided on.  For q = 0 it is 0: the cycle that
+  // ran is not counted and p starts again.
   // Each V-cycle is one launch of a CUDA graph captured once per hierarchy
   // (its buffers never move); without a graph the kernels are launched one by one.
   // Adds the V-cycles to *cycles.  A non-finite residual (the FP32 hierarchy
@@ -1217,7 +1219,13 @@ struct Run {
       ++it;
       if (m.zgraph) cudaGraphLaunch(m.zgraph, st);
       else vcycle(0, true);
-      rc = fine_residual(&res, err);
+      bool q_zero = false;
+      rc = fine_residual(&res, err, &q_zero);
+      if (rc == TBFP_OK && q_zero) {
+        it = 0;
+        k_fill<<<nblk_grid(L.n), kMgThreads, 0, st>>>(L.p, L.n, 0.0f);
+        rc = fine_residual(&res, err);
+      }
     }
     while (rc == TBFP_OK && std::isfinite(res) && it < m.prm.max_iter_mg && res > m.prm.tol_mg) {
       ++it;

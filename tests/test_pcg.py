@@ -192,3 +192,11 @@ def test_coarse_system_keeps_the_scale_of_a_small_domain():
     assert st.iterations == 1
     a, b = O.FField("cl", 1, nx, ny, nz, psi).interior(), ref.interior()
     assert rel_linf(a - a.mean(), b - b.mean()) < 2e-5
+
+
+def test_a_zero_source_takes_no_cycle():
+    """q = 0: the residual is 0 before the first V-cycle, so none is counted and the pressure stays as it was."""
+    g, m, q, beta = _mg_case(32, 32, 16, 0.01, 4)
+    st, psi = _gpu_pcg(g, np.zeros_like(q), beta, 3)
+    assert st.iterations == 0 and st.ms_stage[0] == 0 and st.rel_residual == 0.0
+    assert not psi.any()
