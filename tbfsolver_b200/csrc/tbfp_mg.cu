@@ -498,21 +498,25 @@ __global__ void k_coarse_apply(MgLev L, const double *__restrict__ M, int n1, co
 // The coarse end of a V-cycle, levels l0 .. last, in one launch of one CTA with
 // every level's p, q and beta in shared memory: zero-start smoothing, residual and
 // restriction down to the coarsest level, its bordered inverse applied, then
-// prolongation and smoothing back up.  A launch per step cost 2 to 3 us each, 13 of
-// them for the 16x16x8 and 8x8x4 levels of 256x256x128; the CTA takes 0.039 ms for
-// both.  With the 32x32x16 level in it as well (220 KB) it took 0.188 ms: a sweep of
-// 16,384 cells is too much for one SM.
+// prolongation and smoothing back up.  A launch per step costs 2 to 3 us each, 13 for
+// a smoothed level and the coarsest; one SM saves that as long as a sweep is one round
+// of its threads.  Cycle times in us, in one launch against launch by launch, by the
+// cells of the first level in it (two smoothing iterations each way): 128: 77 / 84,
+// 512: 89 / 101, 768: 91 / 100, 1,024 over 128 and 16: 133 / 149, 1,024: 101 / 102
+// and 142 / 149, 1,152: 104 / 104 and 151 / 152, 1,344: 106 / 104, 1,792: 118 / 108,
+// 2,048: 121 / 110 (a solve of 256x256x128 on six levels: 61.0 / 60.1 ms), 4,096: 138 / 129.
 // q of level l0 comes from the restriction before, p of level l0 and the pending
 // sum of its last smoothing go back to memory.
 // ---------------------------------------------------------------------------
-constexpr int kMgMaxLevels = 16, kTailThreads = 1024;
-constexpr size_t kTailSmem = 64 * 1024;
-constexpr int kTailCoarse = 320;  // unknowns of the coarsest system whose inverse (0.8 MB) one SM applies
+constexpr int kTailThreads = 1024, kTailCells = 1024;  // cells of the first level at most
+// a level has an eighth of the cells of the one before: four levels (1,024, 128, 16, 2)
+// and 128 coarse unknowns at most, 15 KB of shared memory
+constexpr int kTailLevels = 4, kTailCoarse = kTailCells / 8;
 struct MgTail {
   int n;  // levels, the last one the coarsest
   int n_pre, n_post;
-  MgLev L[kMgMaxLevels];
-  const float *beta[kMgMaxLevels];
+  MgLev L[kTailLevels];
+  const float *beta[kTailLevels];
   const float *q0;  // q of the first level
   float *p0;        // its p
   double *post0;    // its pending sum
@@ -534,7 +538,7 @@ __device__ double tail_sum(double v) {  // the same sum in every thread
 __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_constant__ MgTail T) {
   extern __shared__ __align__(16) float ts[];
   const int tid = threadIdx.x, last = T.n - 1;
-  float *p[kMgMaxLevels], *q[kMgMaxLevels], *bt[kMgMaxLevels];
+  float *p[kTailLevels], *q[kTailLevels], *bt[kTailLevels];
   {
     float *f = ts;
     for (int l = 0; l < T.n; ++l) {
@@ -576,7 +580,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_mg_tail(const __grid_consta
     for (int t = tid; t < n; t += kTailThreads) s += P[t];
     return tail_sum(s);
   };
-  double pre[kMgMaxLevels];
+  double pre[kTailLevels];
   for (int l = 0; l < last; ++l) {
     pre[l] = smooth(l, T.n_pre, true);
     // residual of the eight cells under each coarse cell, restricted
@@ -1051,16 +1055,9 @@ int MgSolver::init(const tbfp_mg_params &prm, int nx, int ny, int nz, const doub
     G.py = L.tab + o[13];
     G.pz = L.tab + o[14];
   }
-  // the coarse levels small enough for one SM (k_mg_tail), if the coarsest system
-  // is, and with at least one level to smooth: many SMs apply the inverse faster
+  // the coarse levels small enough for one SM (k_mg_tail), with at least one to smooth
   m.tail = prm.n_levels;
-  size_t tb = 8 * (size_t)m.lv.back().n;
-  for (int l = prm.n_levels - 2; l >= 1 && m.n1 <= kTailCoarse && prm.n_levels - l <= kMgMaxLevels; --l) {
-    tb += 12 * (size_t)m.lv[l].n;
-    if (tb > kTailSmem) break;
-    m.tail = l;
-  }
-  ck(cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
+  for (int l = prm.n_levels - 2; l >= 1 && m.lv[l].n <= kTailCells; --l) m.tail = l;
   // FP64 fine tables from the caller's metrics (the reference's own values)
   std::vector<double> x1(nx), x2(nx), y1(ny), y2(ny), z1(nz), z2(nz);
   for (int i = 0; i < nx; ++i) {
