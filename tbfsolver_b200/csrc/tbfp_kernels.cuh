@@ -179,8 +179,10 @@ int ensemble_blocks_per_sm(size_t smem);
 // The ones with a fused right-hand side + forward x transform, below kRhsFftxMaxM:
 // from 384 on a thread marches two to four columns one after the other at two CTAs
 // per SM, and writing s out and reading it back is faster (1024x512x512: 4.64 ms
-// fused, 2.98 + 1.04 apart; 768x200x256: 0.651 against 0.427 + 0.156), while at 256
-// and below it is slower (512x384x256: 0.680 fused, 0.550 + 0.179 apart).
+// fused, 2.98 + 1.04 apart; 768x200x256: 0.651 against 0.427 + 0.156; in us, thin
+// grids: 768x24x8 17.9 against 3.4 + 6.0, 768x48x16 18.4 against 7.8 + 6.9, 1024x64x32
+// 42.4 against 30.1 + 11.9, 768x64x64 63.7 against 43.7 + 16.8), while at 256 and below
+// it is slower (512x384x256: 0.680 fused, 0.550 + 0.179 apart).
 constexpr int kRhsFftxMaxM = 384;
 #define TBFP_RHS_FFTX_LENGTHS(X) X(4) X(6) X(8) X(12) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256)
 inline bool fft_length_supported(int n) {

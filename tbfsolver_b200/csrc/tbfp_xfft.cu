@@ -9,6 +9,8 @@
 // every kx.  This replaces the pencil transposes of pencilDec.f90:359-562.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "tbfp_kernels.cuh"
 #include "tbfp_stages.cuh"
 
@@ -253,18 +255,20 @@ void launch_mixed_decide(MixedCtl *ctl, const double *acc, double *acc_r, cudaGr
 }
 
 // Split RHS into s on the interior (tbfp_rhs_split and the projection).  Grid
-// (x tiles of 128, y chunks of kRJ rows, nz); a thread owns column (i, k) of a y
+// (x tiles of 128, y chunks of jc rows, nz); a thread owns column (i, k) of a y
 // chunk and walks it in j with 32-bit element offsets, carrying the centre
 // values of 1/rho, psi^n and psi^(n-1) to the next row as its lower y
 // neighbours.  computeSource (poissonEqn.f90:224-253) with computeOldPressDiv
 // (:270-301), nl = 2; divisions by metrics are products with host-computed
 // reciprocals, 1/rho comes from the precomputed array.
 
+constexpr int kRhsBlocks = 6;  // blocks per SM
 template <bool ST>
-__global__ void __launch_bounds__(128, 6) k_rhs(RhsArgs a, GridK g, double *__restrict__ s, Lay Ls) {
+__global__ void __launch_bounds__(128, kRhsBlocks) k_rhs(RhsArgs a, GridK g, double *__restrict__ s, Lay Ls,
+                                                                      int jc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int k = blockIdx.z + 1;
-  const int j0 = blockIdx.y * kRJ + 1, j1 = min(j0 + kRJ - 1, g.ny);
+  const int j0 = blockIdx.y * jc + 1, j1 = min(j0 + jc - 1, g.ny);
   if (i > g.nx) return;  // no block-level barrier in this kernel
   const int pjs = (int)a.Lpsi.sj, pks = (int)a.Lpsi.sk, rjs = (int)a.Lrho.sj, rks = (int)a.Lrho.sk;
   const int xjs = (int)a.Lux.sj, yjs = (int)a.Luy.sj, zjs = (int)a.Luz.sj, zks = (int)a.Luz.sk;
@@ -337,9 +341,16 @@ __global__ void __launch_bounds__(128, 6) k_rhs(RhsArgs a, GridK g, double *__re
 }
 
 void launch_rhs(const RhsArgs &ra, bool has_st, const GridK &g, double *s, Lay Ls, cudaStream_t st) {
-  dim3 grid((g.nx + 127) / 128, (g.ny + kRJ - 1) / kRJ, g.nz);
-  if (has_st) k_rhs<true><<<grid, 128, 0, st>>>(ra, g, s, Ls);
-  else k_rhs<false><<<grid, 128, 0, st>>>(ra, g, s, Ls);
+  // kRJ rows per block, fewer where that leaves less than one round of blocks
+  // (768x24x8: 12.6 us with 32 rows, 3.4 now; 768x48x16: 20.9, 7.8; 1024x64x32:
+  // 35.9, 30.1; 768x64x64, 768 blocks of 32 rows: 43.8, 43.7)
+  const int nbx = (g.nx + 127) / 128;
+  int jc = kRJ;
+  if ((long)nbx * ((g.ny + kRJ - 1) / kRJ) * g.nz < 148L * kRhsBlocks)
+    jc = std::min(kRJ, march_chunk((long)nbx * g.nz, g.ny, 148L * kRhsBlocks, 1));
+  const dim3 grid(nbx, (g.ny + jc - 1) / jc, g.nz);
+  if (has_st) k_rhs<true><<<grid, 128, 0, st>>>(ra, g, s, Ls, jc);
+  else k_rhs<false><<<grid, 128, 0, st>>>(ra, g, s, Ls, jc);
 }
 
 // ---------------------------------------------------------------------------

@@ -97,9 +97,9 @@ def test_epsilon_pivot_against_exact_gauge_on_the_projection_chain():
 @pytest.mark.parametrize("nx", [768, 1024])
 def test_long_x_rows_against_the_c_oracle(nx):
     """nx = 768 and 1024 (half-length transforms of 384 and 512 points): the
-    fused right-hand side then gives each thread two to four columns of a row,
-    and the x transforms run at two CTAs per SM.  One projection on a thin
-    channel against the C restatement, same bar as the benchmarked sizes."""
+    right-hand side runs apart from the x transform there, and the x transforms
+    at two CTAs per SM.  One projection on a thin channel against the C
+    restatement, same bar as the benchmarked sizes."""
     from tbfsolver_b200.solver import PoissonEqn
 
     spec = synth.small_spec(nx, 24, 8, stretched=True, nbubbles=2, radius=0.3, rhog=0.05)
@@ -121,3 +121,41 @@ def test_long_x_rows_against_the_c_oracle(nx):
     for f, want in zip(uo.components(), wu):
         assert rel_linf(Field.like(f, host(f)).interior(), Field.like(f, want).interior()) < TOL_P, f.kind
     assert abs(st.max_div - md_ref) < TOL_DIV
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(512, 25, 8), (768, 25, 8), (1024, 7, 4), (1024, 33, 64)])
+@pytest.mark.parametrize("tension", [False, True])
+def test_long_x_rows_and_both_forms_of_the_right_hand_side(dims, tension):
+    """nx = 512, where a thread of the fused right-hand side marches two columns, and the lengths from 768 on, where
+    it runs apart: rows per block of one, two and the full 32, each with a remainder, with and without surface
+    tension.  One projection against the oracle, same bar."""
+    from tbfsolver_b200.fields import VField
+    from tbfsolver_b200.solver import PoissonEqn
+
+    nx, ny, nz = dims
+    spec = synth.small_spec(nx, ny, nz, stretched=True, nbubbles=2, radius=0.3, rhog=0.05)
+    inp = synth.make_inputs(spec, seed=32)
+    g, rng = inp.grid, np.random.default_rng(nx + ny)
+    st = [[O.FField(k, 1, nx, ny, nz, 0.01 * rng.standard_normal(Field(k, 1, nx, ny, nz).a.shape))
+           for k in ("sx", "sy", "sz")] for _ in range(2)] if tension else [None, None]
+    if tension:
+        for f in st:
+            O.equate_periodic_bc(f[0], f[2])             # periodic duplicate faces
+            f[1].a[:, 1, :] = f[1].a[:, -2, :] = 0.0  # no force on the wall faces
+    ref = O.projection(mesh_of(g), *[to_oracle(f, g) for f in (*inp.u.components(), inp.rho, inp.psi_n, inp.psi_nm1)],
+                       inp.dt, inp.alpha, inp.rho0, *st)
+    cu = lambda f: Field(f.kind, f.hd, nx, ny, nz, torch.as_tensor(f.a).cuda())  # noqa: E731
+    eqn = PoissonEqn(g, spec.rhol, spec.rhog)
+    try:
+        psi = cu(inp.psi_n)
+        u = VField(*[cu(f) for f in inp.u.components()])
+        uo = VField(*[Field.like(f, torch.zeros_like(f.a)) for f in u.components()])
+        extra = [[cu(f) for f in fs] for fs in st] if tension else []
+        torch.cuda.synchronize()
+        eqn.projection(psi, cu(inp.psi_n), cu(inp.psi_nm1), cu(inp.rho), u, inp.dt, inp.alpha, *extra, u_out=uo)
+    finally:
+        eqn.close()
+    assert rel_linf(psi.a.cpu().numpy(), ref.psi.a) < TOL_P
+    for f, r in zip(uo.components(), (ref.ux, ref.uy, ref.uz)):
+        assert rel_linf(Field.like(f, f.a.cpu().numpy()).interior(), r.interior()) < TOL_P
