@@ -60,7 +60,9 @@ __device__ __forceinline__ double face_flux(double q, double vm, double vc, doub
   if (S == 0 || (S == 5 && !sh)) return __dmul_rn(q, a + 0.5 * d);
   const double n = a - (up ? vm : vpp);
   if constexpr (S == 2) return __dmul_rn(q, d == 0.0 ? a : a + 0.125 * (n + 3.0 * d));
-  const bool same = n * d > 0.0;
+  // n has d's sign: n with its sign flipped where d is negative is above 0 (the product
+  // n * d underflows where both are below 1e-162)
+  const bool same = __hiloint2double(__double2hiint(n) ^ (__double2hiint(d) & (int)0x80000000u), __double2loint(n)) > 0.0;
   if constexpr (S == 3) return __dmul_rn(q, same ? a + n * (d / (n + d)) : a);
   const double an = fabs(n), ad = fabs(d);
   const double lo = an < ad ? an : ad, hi = an < ad ? ad : an;

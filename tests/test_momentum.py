@@ -390,3 +390,28 @@ def test_out_of_place_predictor_matches_the_oracle_at_tile_edges(scheme, dims):
             assert rel_linf(_host(got), want.a) < 1e-13
         for got, want in zip(mom.fluxes(), phi):
             assert rel_linf(got, want) < 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scheme", [2, 3, 4, 5])
+def test_limiters_keep_a_velocity_whose_differences_have_no_product(scheme):
+    """ux of about 1e-170 convected by uy and uz of ordinary size: the product of two of its differences is below
+    the smallest double, so a limiter that compares their signs by it would fall back to upwind.  mu = 0 leaves
+    the convection alone in phi_x.  Bar as above."""
+    nx, ny, nz = 32, 10, 12
+    g = _grid(nx, ny, nz, True)
+    u = _velocity(g, 40 + scheme)
+    u[0].a *= 2.0 ** -565
+    c, mu, rho = _props(g, 8)
+    mu.a[...] = 0.0
+    with FastPoissonSolver(g, hd_u=HD_U, hd_rho=HD_RHO, hd_st=HD_ST) as fps:
+        mom = MomentumEqn(fps, scheme=scheme)
+        du = VField(*[_to_dev(f, "device") for f in u])
+        dc, dmu, drho = (_to_dev(f, "device") for f in (c, mu, rho))
+        torch.cuda.synchronize()
+        mom.predictor(du, dc, dmu, drho, dt=1e-3, alpha=1.0, gamma=1.5, xi=-0.5, rho0=0.02)
+        got = mom.fluxes()
+    want = O.momentum_fluxes(mesh_of(g), *u, c, mu, rho, scheme)
+    assert 0.0 < np.max(np.abs(want[0])) < 1e-165
+    for a, b in zip(got, want):
+        assert rel_linf(a, b) < 1e-12
