@@ -39,9 +39,11 @@ __device__ __forceinline__ bool sharp_cell(double cxp, double cxm, double cyp, d
 // r = (vc - vm)/(vp - vc), and B its mirror image (momentumEqn.f90:240-256 and
 // the like; limiters :611-734).  One of the products is always zero, so only
 // the upwind side is evaluated: a the upwind value, f the one behind it, d the
-// difference across the face, n = a - f, r = n/d.  (An infinity or NaN on the
-// other side's far value then stays out of this face; it is in the face beside
-// it.)  psi(r) d is written without the ratio:
+// difference across the face, n = a - f, r = n/d.  The other side's product is
+// zero times its value, and NaN where that is not finite: with van Leer's limiter if
+// its far value h makes its ratio +infinity (psi = inf/inf), with QUICK if h is not
+// finite (far_cell, far_face), never with superbee.  psi(r) d is written without the
+// ratio:
 //   QUICK     (r+3)/4 d            = (n + 3d)/4, and 0 for d = 0 (the reference's
 //                                    approx_zero makes it so)
 //   van Leer  (r+|r|)/(1+|r|) d    = 2 n d/(n + d) for n, d of one sign, else 0
@@ -62,12 +64,44 @@ __device__ __forceinline__ double face_flux(double q, double vm, double vc, doub
   if constexpr (S == 2) return __dmul_rn(q, d == 0.0 ? a : a + 0.125 * (n + 3.0 * d));
   // n has d's sign: n with its sign flipped where d is negative is above 0 (the product
   // n * d underflows where both are below 1e-162)
-  const bool same = __hiloint2double(__double2hiint(n) ^ (__double2hiint(d) & (int)0x80000000u), __double2loint(n)) > 0.0;
-  if constexpr (S == 3) return __dmul_rn(q, same ? a + n * (d / (n + d)) : a);
+  const int ds = __double2hiint(d) & (int)0x80000000u;
+  const bool same = __hiloint2double(__double2hiint(n) ^ ds, __double2loint(n)) > 0.0;
+  if constexpr (S == 3) {
+    // h infinite and of d's sign: (h minus the downwind value)/d is +infinity
+    // (512x384x256: 3.36 -> 3.43 ms; looked at once per cell 3.70)
+    const bool wild = (__double2hiint(up ? vpp : vm) ^ ds) == 0x7ff00000;
+    const double x = __dmul_rn(q, same ? a + n * (d / (n + d)) : a);
+    return wild ? __longlong_as_double(0x7ff8000000000000LL) : x;
+  }
   const double an = fabs(n), ad = fabs(d);
   const double lo = an < ad ? an : ad, hi = an < ad ? ad : an;
   const double m = 2.0 * lo < hi ? lo : 0.5 * hi;  // half of |psi(r) d|
   return __dmul_rn(q, same ? a + copysign(m, d) : a);
+}
+
+// QUICK's NaN from the values two cells away, whichever side the wind comes from.
+// The high word of an infinite or NaN double (or one beyond 1e306) is a float that is
+// not finite, so zero times it, one instruction a value, is NaN, else zero; or'ed
+// into the high word of a flux it makes that NaN or leaves it.  512x384x256: 2.30 ->
+// 2.34 ms; as zero times the far value in every face's formula 2.45, behind a branch
+// on the float 2.67.
+__device__ __forceinline__ float far_term(double v, float s) {
+  return __fmaf_rn(0.0f, __int_as_float(__double2hiint(v)), s);
+}
+__device__ __forceinline__ double or_nan(double x, float s) {
+  return __hiloint2double(__double2hiint(x) | __float_as_int(s), __double2loint(x));
+}
+// f: a flux difference of the cell with the neighbours c(+-2, 0), c(0, +-2) in x and y
+template <int S, class Val>
+__device__ __forceinline__ double far_cell(double f, const Val &c) {
+  if constexpr (S != 2) return f;
+  return or_nan(f, far_term(c(0, 2), far_term(c(0, -2), far_term(c(2, 0), far_term(c(-2, 0), 0.0f)))));
+}
+// f: the flux of the face whose far values are vm and vpp
+template <int S>
+__device__ __forceinline__ double far_face(double f, double vm, double vpp) {
+  if constexpr (S != 2) return f;
+  return or_nan(f, far_term(vpp, far_term(vm, 0.0f)));
 }
 
 struct MomArgs {
@@ -252,7 +286,8 @@ __device__ __forceinline__ double F_xy(const Acc &A, bool sh = true) {
 template <int S, class Acc>
 __device__ __forceinline__ double F_xz(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (w(0, 0, 0) + w(1, 0, 0)), u(0, 0, -1), u(0, 0, 0), u(0, 0, 1), u(0, 0, 2), sh);
+  const double f = face_flux<S>(0.5 * (w(0, 0, 0) + w(1, 0, 0)), u(0, 0, -1), u(0, 0, 0), u(0, 0, 1), u(0, 0, 2), sh);
+  return far_face<S>(f, u(0, 0, -1), u(0, 0, 2));
 }
 // uy faces
 template <int S, class Acc>
@@ -269,8 +304,9 @@ __device__ __forceinline__ double F_yy(const Acc &A, bool sh = true) {
 template <int S, class Acc>
 __device__ __forceinline__ double F_yz(const Acc &A, const Met &g, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (w(0, 1, 0) * g.dyf1 + w(0, 0, 0) * g.dyf0) * g.ryc1, v(0, 0, -1), v(0, 0, 0), v(0, 0, 1),
+  const double f = face_flux<S>(0.5 * (w(0, 1, 0) * g.dyf1 + w(0, 0, 0) * g.dyf0) * g.ryc1, v(0, 0, -1), v(0, 0, 0), v(0, 0, 1),
                       v(0, 0, 2), sh);
+  return far_face<S>(f, v(0, 0, -1), v(0, 0, 2));
 }
 // uz faces
 template <int S, class Acc>
@@ -286,7 +322,8 @@ __device__ __forceinline__ double F_zy(const Acc &A, bool sh = true) {
 template <int S, class Acc>
 __device__ __forceinline__ double F_zz(const Acc &A, bool sh = true) {
   TBFP_MOM_ACCESSORS;
-  return face_flux<S>(0.5 * (w(0, 0, 0) + w(0, 0, 1)), w(0, 0, -1), w(0, 0, 0), w(0, 0, 1), w(0, 0, 2), sh);
+  const double f = face_flux<S>(0.5 * (w(0, 0, 0) + w(0, 0, 1)), w(0, 0, -1), w(0, 0, 0), w(0, 0, 1), w(0, 0, 2), sh);
+  return far_face<S>(f, w(0, 0, -1), w(0, 0, 2));
 }
 
 // x component at face (i, j, k) (momentumEqn.f90:228-341) from the convective
@@ -372,9 +409,10 @@ template <int S, bool Z, class Acc>
 __device__ __forceinline__ double phi_x(const Acc &A, const Met &g, double invrho, double cz) {
   TBFP_MOM_ACCESSORS;
   const bool sh = sharp_cell<S>(c(1, 0, 0), c(0, 0, 0), c(0, 1, 0), c(0, -1, 0), c(0, 0, 1), c(0, 0, -1));
-  const double cx = F_xx<S>(A, sh) - F_xx<S>(A.shifted(-1, 0), sh);
+  double cx = F_xx<S>(A, sh) - F_xx<S>(A.shifted(-1, 0), sh);
   const double cy = F_xy<S>(A, sh) - F_xy<S>(A.shifted(0, -1), sh);
   if constexpr (Z) cz = F_xz<S>(A, sh) - F_xz<S>(A.down(), sh);
+  cx = far_cell<S>(cx, [&](int di, int dj) { return u(di, dj, 0); });
   return tail_x(A, g, invrho, cx, cy, cz);
 }
 
@@ -382,9 +420,10 @@ template <int S, bool Z, class Acc>
 __device__ __forceinline__ double phi_y(const Acc &A, const Met &g, double invrho, double cz) {
   TBFP_MOM_ACCESSORS;
   const bool sh = sharp_cell<S>(c(1, 0, 0), c(-1, 0, 0), c(0, 1, 0), c(0, 0, 0), c(0, 0, 1), c(0, 0, -1));
-  const double cx = F_yx<S>(A, g, sh) - F_yx<S>(A.shifted(-1, 0), g, sh);
+  double cx = F_yx<S>(A, g, sh) - F_yx<S>(A.shifted(-1, 0), g, sh);
   const double cy = F_yy<S>(A, sh) - F_yy<S>(A.shifted(0, -1), sh);
   if constexpr (Z) cz = F_yz<S>(A, g, sh) - F_yz<S>(A.down(), g, sh);
+  cx = far_cell<S>(cx, [&](int di, int dj) { return v(di, dj, 0); });
   return tail_y(A, g, invrho, cx, cy, cz);
 }
 
@@ -392,9 +431,10 @@ template <int S, bool Z, class Acc>
 __device__ __forceinline__ double phi_z(const Acc &A, const Met &g, double invrho, double cz) {
   TBFP_MOM_ACCESSORS;
   const bool sh = sharp_cell<S>(c(1, 0, 0), c(-1, 0, 0), c(0, 1, 0), c(0, -1, 0), c(0, 0, 1), c(0, 0, 0));
-  const double cx = F_zx<S>(A, sh) - F_zx<S>(A.shifted(-1, 0), sh);
+  double cx = F_zx<S>(A, sh) - F_zx<S>(A.shifted(-1, 0), sh);
   const double cy = F_zy<S>(A, sh) - F_zy<S>(A.shifted(0, -1), sh);
   if constexpr (Z) cz = F_zz<S>(A, sh) - F_zz<S>(A.down(), sh);
+  cx = far_cell<S>(cx, [&](int di, int dj) { return w(di, dj, 0); });
   return tail_z(A, g, invrho, cx, cy, cz);
 }
 #undef TBFP_MOM_ACCESSORS
@@ -409,10 +449,10 @@ constexpr int kMomBlocks = 2;  // blocks per SM
 // the step before the one that computes on it.
 // Bound: FP64 latency and instructions at 16 warps per SM (registers and the
 // plane rings allow two blocks).  512x384x256, out of place, by scheme 0..5:
-// 2.25 2.17 2.32 3.48 2.68 3.02 ms, where limiters evaluated on both sides of each
+// 2.11 2.02 2.34 3.43 2.57 2.78 ms, where limiters evaluated on both sides of each
 // face, three reciprocals of rho per cell, the last step's fluxes loaded where
-// they are used, and lower z faces evaluated again took 3.06 3.07 3.29 8.97 5.21
-// 4.15 ms.  Three blocks per SM (80 registers) spill: 3.76 ms for QUICK.  Each x
+// they are used, and lower z faces evaluated again took 2.92 2.92 3.14 8.82 5.07
+// 3.80 ms.  Three blocks per SM (80 registers) spill: 3.76 ms for QUICK.  Each x
 // and y face computed once per tile (shared memory and a barrier) does not pay
 // any more: 3.68 against 3.56 ms for van Leer's limiter, the dearest.
 template <int S, bool OUT>

@@ -415,3 +415,30 @@ def test_limiters_keep_a_velocity_whose_differences_have_no_product(scheme):
     assert 0.0 < np.max(np.abs(want[0])) < 1e-165
     for a, b in zip(got, want):
         assert rel_linf(a, b) < 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scheme, bad", [(s, np.inf) for s in range(6)] + [(s, -np.inf) for s in range(6)]
+                         + [(s, np.nan) for s in range(3)])
+def test_a_non_finite_velocity_reaches_the_fluxes_of_the_formula(scheme, bad):
+    """max(q,0)*A + min(q,0)*B takes in the far value of both sides, whichever side the wind comes from: an
+    infinity (and, where no limiter's max(0, r) drops it, a NaN) makes the same fluxes non-finite as in the
+    oracle's restatement, two cells away as well, for each component that holds it."""
+    nx, ny, nz = 32, 12, 12
+    g = _grid(nx, ny, nz, True)
+    m = mesh_of(g)
+    c, mu, rho = _props(g, 8)
+    with FastPoissonSolver(g, hd_u=HD_U, hd_rho=HD_RHO, hd_st=HD_ST) as fps:
+        mom = MomentumEqn(fps, scheme=scheme)
+        dc, dmu, drho = (_to_dev(f, "device") for f in (c, mu, rho))
+        for comp in range(3):
+            u = _velocity(g, 50 + comp)
+            u[comp].v(14, 14, 6, 6, 5, 5)[...] = bad
+            du = VField(*[_to_dev(f, "device") for f in u])
+            torch.cuda.synchronize()
+            mom.predictor(du, dc, dmu, drho, dt=1e-3, alpha=1.0, gamma=1.5, xi=-0.5, rho0=0.02)
+            with np.errstate(invalid="ignore"):
+                want = O.momentum_fluxes(m, *u, c, mu, rho, scheme)
+            for a, b in zip(mom.fluxes(), want):
+                assert not np.isfinite(b).all()
+                assert np.array_equal(np.isfinite(a), np.isfinite(b))
