@@ -120,13 +120,16 @@ def _widen(f: Field, hd: int) -> Field:
 
 
 @pytest.mark.gpu
-def test_projection_with_wider_halos_matches_default_halos():
+@pytest.mark.parametrize("limit", [None, 5_000_000_000])
+def test_projection_with_wider_halos_matches_default_halos(limit):
     """The out-of-place projection with psi and rho halos of 2 and velocity
     halos of 3 against the same projection with the default halos (1 and 2).
     Odd and even halos shift the tensor-map boxes of the staged correction by
     one column (the 16-byte start rule), so both offsets of every box run here;
     x tiles of 128 with a partial last tile, ny not a multiple of the tile
-    height.  The arithmetic is the same, so the interiors agree to the bit."""
+    height.  The arithmetic is the same, so the interiors agree to the bit.
+    The grid is below the staged form's size: a wait limit of the caller's own
+    asks for it, the default takes the kernel form."""
     spec = synth.small_spec(192, 20, 12, stretched=True, nbubbles=2, radius=0.3, rhog=0.05)
     inp = synth.make_inputs(spec, seed=13, device="cuda")
     g = inp.grid
@@ -139,6 +142,8 @@ def test_projection_with_wider_halos_matches_default_halos():
         uo = VField(*[Field.like(f, torch.zeros_like(f.a)) for f in u.components()])
         eqn = PoissonEqn(g, spec.rhol, spec.rhog, hd_psi=hps, hd_rho=hps, hd_u=hu)
         try:
+            if limit is not None:
+                eqn.solver.set_wait_limit(limit)
             st = eqn.projection(psi, pn, pnm1, rho, u, inp.dt, inp.alpha, u_out=uo)
         finally:
             eqn.close()

@@ -26,22 +26,29 @@ def _clone_u(u):
     return VField(*[Field.like(f, f.a.clone()) for f in u.components()])
 
 
+# A wait limit of the caller's own (longer than the default): grids as small as these
+# take the staged form of the velocity correction with it, the kernel form without.
+LONG_WAIT = 5_000_000_000
+
+
 def _poison(t: torch.Tensor, value: float, where: float = 0.37):
     flat = t.view(-1)
     flat[int(where * flat.numel())] = value
 
 
-@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("precision, limit", [("fp64", None), ("fp64", LONG_WAIT), ("mixed", None)])
 # (rho = Inf is not in the list: 1/rho = 0 is a finite inverse density and every
 # coefficient stays finite, so there is nothing to report; rho = 0 makes 1/rho
 # infinite and must be reported)
 @pytest.mark.parametrize("field,value", [("ux", float("nan")), ("uz", float("inf")), ("rho", float("nan")),
                                          ("rho", 0.0), ("psi_n", float("nan"))])
-def test_projection_reports_nonfinite_inputs(precision, field, value):
+def test_projection_reports_nonfinite_inputs(precision, limit, field, value):
     spec, inp = _inputs()
     g = inp.grid
     eqn = PoissonEqn(g, spec.rhol, spec.rhog, precision=precision, tol=1e-10, max_iter=6)
     try:
+        if limit is not None:
+            eqn.solver.set_wait_limit(limit)
         u = _clone_u(inp.u)
         rho = Field.like(inp.rho, inp.rho.a.clone())
         pn = Field.like(inp.psi_n, inp.psi_n.a.clone())
@@ -108,8 +115,9 @@ def test_correction_copy_wait_limit_reports_a_timeout():
     """The staged correction bounds each wait for the bulk copies of its input
     planes.  With the bound at zero cycles a copy that has not landed at the
     first look counts as late: the kernel lets its copies in flight land, ends,
-    and the call returns TBFP_ETIMEOUT (not a divergence error).  With the
-    default bound restored the same handle gives the same answer as before."""
+    and the call returns TBFP_ETIMEOUT (not a divergence error).  With a long
+    bound again the same handle gives the same answer as before, and so does the
+    default bound's form without copies."""
     from tbfsolver_b200._native import TBFP_ETIMEOUT
 
     spec, inp = _inputs()
@@ -123,16 +131,18 @@ def test_correction_copy_wait_limit_reports_a_timeout():
         return [psi.a.clone()] + [f.a.clone() for f in uo.components()], st.max_div
 
     try:
+        eqn.solver.set_wait_limit(LONG_WAIT)
         want, md = run()
         eqn.solver.set_wait_limit(0)
         with pytest.raises(TbfpError) as ei:
             run()
         assert ei.value.code == TBFP_ETIMEOUT
-        eqn.solver.set_wait_limit(4_000_000_000)
-        got, md2 = run()
-        assert md2 == md
-        for a, b in zip(want, got):
-            assert torch.equal(a, b)
+        for limit in (LONG_WAIT, 4_000_000_000):
+            eqn.solver.set_wait_limit(limit)
+            got, md2 = run()
+            assert md2 == md
+            for a, b in zip(want, got):
+                assert torch.equal(a, b)
         with pytest.raises(TbfpError):
             eqn.solver.set_wait_limit(-1)
     finally:
