@@ -424,8 +424,9 @@ bool encode_rows(CUtensorMap *m, const double *base, const Lay &Ly, long nk) {
 constexpr int kMinChunk = 8;
 // Tiles x chunks below which the kernel form is faster: a CTA's march of at least
 // kMinChunk planes takes 21 us however few CTAs there are (32x24x16: 21.2 against
-// 3.7 us; 96x100x48, 78 CTAs: 21.9 against 14.2; 128x128x64, 128 CTAs: 23.0
-// against 25.3; 256x256x128: 152 against 187).
+// 3.7 us; 96x100x48, 78 CTAs: 21.9 against 14.2; 128x96x64 and 256x96x32, 96 CTAs:
+// 22.6 against 19.1 and 19.6; 128x128x64, 128 CTAs: 23.0 against 25.3; 256x256x128:
+// 152 against 187).
 constexpr int kFewCtas = 100;
 
 // planes per chunk: the chunk count that best fills whole waves of one CTA

@@ -32,7 +32,7 @@
 //   3. k_st_faces: the faces of the listed cells and their periodic images.
 // Bound: HBM for the first (33 bytes per cell: c 8, class 1, st 24), loads and
 // instructions per interface cell for the others.
-// 512x384x256 with 200 bubbles: 0.289 + 0.169 + 0.041 ms (the first at 5.7 TB/s),
+// 512x384x256 with 200 bubbles: 0.289 + 0.173 + 0.041 ms (the first at 5.7 TB/s),
 // where dense passes over all cells (classes with a copy of c, curvature, faces)
 // took 0.44 + 10.6 + 2.09 ms.
 // The decisions (the normal's ranking, the column sums) use adds and multiplies
@@ -191,7 +191,8 @@ __device__ __forceinline__ double face_pos(const StGrid &g, int d, int q) {
 // decision.  Bound: instructions of the columns and L1 misses on c's rows; one
 // thread per grid cell with serial walks took 10.6 ms on 512x384x256 (0.9 % of
 // the lanes busy), three cells per warp with the formula repeated by nine lanes
-// 1.29 ms, this form 0.169 ms.
+// 1.29 ms, this form 0.173 ms (0.169 with a cell's nine columns at once, which walks
+// the eight in vain where its own is not valid).
 constexpr int kCurvWarps = 4;
 constexpr int kCurvBlocks = 6;  // blocks per SM
 __global__ void __launch_bounds__(32 * kCurvWarps, kCurvBlocks) k_st_curvature(const double *__restrict__ c, Lay Lc,
