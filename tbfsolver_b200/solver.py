@@ -151,7 +151,8 @@ class FastPoissonSolver:
     def set_wait_limit(self, cycles: int) -> None:
         """Bound, in SM clock cycles, on each wait of the velocity correction for the copies
         that stage its inputs (tbfp_set_wait_limit; default 4e9, about 2 s).  A wait that runs
-        out makes the projection raise TbfpError with TBFP_ETIMEOUT; the handle stays usable."""
+        out makes the projection raise TbfpError with TBFP_ETIMEOUT; the handle stays usable.
+        Small grids stage nothing at the default bound and the copies at any other."""
         check(self.lib.tbfp_set_wait_limit(self.h, int(cycles)), self.h)
 
     # --- solveFPS ----------------------------------------------------------
